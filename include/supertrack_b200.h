@@ -163,10 +163,11 @@ ST_API st_status st_measure_smem_atomic_peak(st_ctx* ctx, double* atomics_per_se
 /* Tuning knobs: target deposit*oversamples per work item, resident CTAs (0 = one per SM). */
 ST_API st_status st_ctx_set_tuning(st_ctx* ctx, int64_t item_cost, int32_t grid);
 /* Named work-planning parameters (all take effect at the next run):
- *   item_cost          deposit*oversamples per private work item            (default 262144)
+ *   item_cost          deposit*oversamples per private work item, at most   (default 262144)
  *   grid               resident CTAs of the fused kernel, 0 = one per SM     (default 0)
  *   chunk_windows      windows of 8192 kept deposits per chunk of a shared unit   (default 4)
- *   max_helpers        helper items per shared unit                          (default 32)
+ *   max_helpers        helper items per shared unit; most items that one oversample of a job
+ *                      in layer windows is split into                        (default 32)
  *   share_divisor      a job runs as shared units (one per oversample) when its kept deposits
  *                      exceed batch units / (share_divisor * grid); 0 = never (default 8)
  *   shared_min_chunks  ... and exceed this many chunks                       (default 4)
@@ -180,12 +181,14 @@ ST_API st_status st_ctx_set_tuning(st_ctx* ctx, int64_t item_cost, int32_t grid)
  *                      oversample): side 2d when its deposits per sphere diameter of track
  *                      length, n * d / (2 HL), times its oversamples are at most this; 0 = side
  *                      d for every job. Results do not depend on it          (default 25000)
- *   sort_deposits      prepare blocks (1024 source deposits) that write their kept deposits
- *                      grouped by d-cell, the groups in the order of their first deposit, so
- *                      that deposits of one sphere arrive together in the fused kernel: 0 none
- *                      (source order), 1 the blocks of jobs with window boundary flags (dense
- *                      multi-window tracks), 2 all. Results do not depend on it (sums are
- *                      exact)                                                (default 1)
+ *   sort_deposits      order of the kept deposits: 0 source order. 1: the jobs that qualify for
+ *                      window boundary flags (see flag_min_kept) are ordered by z layer instead
+ *                      and run in windows of whole layers, which share no sphere (a track across
+ *                      z, with most deposits in a few layers, keeps the flags); their prepare
+ *                      blocks (1024 source deposits) write their kept deposits grouped by
+ *                      d-cell, so that deposits of one sphere arrive together in the fused
+ *                      kernel. 2: the blocks of all other jobs are grouped too. Results do not
+ *                      depend on it (sums are exact)                         (default 1)
  *   precision          64 = the reference's FP64 arithmetic; 32 = FP32 geometry variant: x, y,
  *                      shifts, the x/y box test, x/y lattice index and sphere distance in float
  *                      (z, keys and energies as in FP64). No reference counterpart: the

@@ -18,6 +18,7 @@ namespace st {
 cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_flagged,
                            cudaStream_t s);
 cudaError_t configure_fused();
+bool fused_big_table(int max_nbins, int table_slots);
 cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s);
 cudaError_t launch_fp64_probe(double* out, int blocks, int iters, cudaStream_t s);
 cudaError_t launch_unit_wait_probe(int* table, int* error_flags, int* out, long long max_polls,
@@ -143,6 +144,7 @@ struct st_ctx {
   DevBuf pxy, pdz2, pv, pkey;
   DevBuf d_jobs, d_aux, d_hists, d_items, d_blk, d_counter, d_err, d_blk_count, d_blk_off, d_blk_job;
   DevBuf c_cells, pz;               // cell arena and shifted z of flagged jobs
+  DevBuf z_bins, z_wins;            // z bins and window lists of layered jobs
   DevBuf u_next, u_done, u_table, pool;  // shared units and the spill-table pool
   DevBuf d_plan, d_plan_misc;             // planner: per-job plans and scratch counters
   DevBuf g_keys, g_lo, g_hi, g_used, g_count;
@@ -196,6 +198,7 @@ struct st_ctx {
   int64_t cache_arena_total = 0;
   int cache_max_nbins = 0;
   int64_t cache_cells = 0;
+  int64_t cache_bins = 0;
   bool cache_any_flagged = false;
   int64_t cache_units = 0;
   int64_t cache_item_cap = 0;
@@ -319,8 +322,15 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
 
   std::vector<JobDev> jd(nj);
   std::vector<int64_t> blk(nj + 1, 0);
-  int64_t cells_total = 0;
+  int64_t cells_total = 0, bins_total = 0, wins_total = 0;
   bool any_flagged = false;
+  // layer windows of two warp tiles per warp, one on the table of half the slots
+  int max_nbins = 0;
+  for (size_t i = 0; i < nj; ++i)
+    max_nbins = std::max(max_nbins, c->hists[c->jobs[first + i].desc.hist_id].nbins);
+  c->cache_max_nbins = max_nbins;
+  const int win_tiles = st::fused_big_table(max_nbins, c->table_slots)
+                            ? st::kWinTiles * st::kFusedWarps : st::kFusedWarps;
   for (size_t i = 0; i < nj; ++i) {
     JobHost& J = c->jobs[first + i];
     JobDev& D = jd[i];
@@ -384,6 +394,19 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
       cells_total += D.cell_cap;
       any_flagged = true;
     }
+    // z bins: one per lattice layer, or per 2^k layers on a lattice of more than kMaxBins
+    D.bin_off = bins_total;
+    D.win_off = wins_total;
+    D.n_bins = 0;
+    D.bin_shift = 0;
+    D.layers = (D.flagged && c->sort_deposits >= 1 && J.track.n < ((int64_t)1 << 31)) ? 1 : 0;
+    D.reserved = 0;
+    if (D.layers) {
+      while (((D.N - 1) >> D.bin_shift) >= (uint32_t)st::kMaxBins) ++D.bin_shift;
+      D.n_bins = (int32_t)((D.N - 1) >> D.bin_shift) + 1;
+      bins_total += D.n_bins;
+      wins_total += st::window_cap(J.track.n, (int64_t)win_tiles * st::kWarpTile);
+    }
     blk[i + 1] = blk[i] + (J.n_pad + st::kPrepSlotsPerBlock - 1) / st::kPrepSlotsPerBlock;
   }
   std::vector<HistDev> hd(c->hists.size());
@@ -404,11 +427,6 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
       hd[h].cb = c->hists[h].nbins / (hi - lo);
     }
   }
-  int max_nbins = 0;
-  for (size_t i = 0; i < nj; ++i)
-    max_nbins = std::max(max_nbins, c->hists[c->jobs[first + i].desc.hist_id].nbins);
-  c->cache_max_nbins = max_nbins;
-
   // work items are planned on the device from the kept counts (k_plan_*); here only their
   // capacity: every job as shared units with the most helpers is the upper bound
   int64_t total_os = 0, work_jobs = 0;
@@ -434,6 +452,8 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   ST_CUDA(ensure(c->d_blk_count, (size_t)blk[nj] * 4), "prepare block counts");
   ST_CUDA(ensure(c->d_blk_job, (size_t)std::max<int64_t>(1, blk[nj]) * 4), "prepare block jobs");
   ST_CUDA(ensure(c->c_cells, (size_t)cells_total * sizeof(st::CellSlot)), "cell arena");
+  ST_CUDA(ensure(c->z_bins, (size_t)bins_total * 4), "z bins");
+  ST_CUDA(ensure(c->z_wins, (size_t)wins_total * 8), "window lists");
   ST_CUDA(ensure(c->pz, any_flagged ? (size_t)prep_total * 8 : 16), "shifted z");
   ST_CUDA(ensure(c->d_blk_off, (size_t)blk[nj] * 8), "prepare block offsets");
   ST_CUDA(ensure(c->d_counter, 16), "work counter");
@@ -508,6 +528,10 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   pp.blk_count = (int32_t*)c->d_blk_count.p;
   pp.blk_offset = (int64_t*)c->d_blk_off.p;
   pp.cells = (st::CellSlot*)c->c_cells.p;
+  pp.bins = (uint32_t*)c->z_bins.p;
+  pp.wins = (unsigned long long*)c->z_wins.p;
+  pp.win_tiles = win_tiles;
+  pp.any_flags = (int32_t*)((char*)c->d_counter.p + 8);
   pp.PZ = (double*)c->pz.p;
   pp.PXY = (double2*)c->pxy.p;
 
@@ -543,6 +567,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   fp.unit_done = (unsigned int*)c->u_done.p;
   fp.unit_table = (int*)c->u_table.p;
   fp.pool_bits = (unsigned int*)c->pool.p;
+  fp.wins = pp.wins;
   fp.chunk_windows = c->chunk_windows;
   fp.fp32 = pp.fp32;
 
@@ -554,6 +579,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   c->cache_item_cap = item_cap;
   c->cache_arena_total = arena_total;
   c->cache_cells = cells_total;
+  c->cache_bins = bins_total;
   c->cache_any_flagged = any_flagged;
   c->cache_units = units;
   // planner parameters; the scratch block holds total_units (8 B), n_items (4 B), the unit
@@ -601,9 +627,8 @@ st_status enqueue_run(st_ctx* c, const st::FusedParams& fp, size_t nj, bool want
     ST_CUDA(cudaMemsetAsync(c->u_done.p, 0, (size_t)c->cache_units * 4, c->stream), "unit reset");
     ST_CUDA(cudaMemsetAsync(c->u_table.p, 0xFF, (size_t)c->cache_units * 4, c->stream), "unit reset");
   }
-  if (c->cache_cells > 0) {
-    ST_CUDA(cudaMemsetAsync(c->c_cells.p, 0xFF, (size_t)c->cache_cells * sizeof(st::CellSlot), c->stream), "cell reset");
-  }
+  if (c->cache_bins > 0)
+    ST_CUDA(cudaMemsetAsync(c->z_bins.p, 0, (size_t)c->cache_bins * 4, c->stream), "z bin reset");
   ST_CUDA(cudaMemsetAsync(c->d_err.p, 0, 16, c->stream), "reset errors");
   if (want_export) ST_CUDA(cudaMemsetAsync(c->ex_count.p, 0, 16, c->stream), "export counter");
 
@@ -634,9 +659,8 @@ st_status enqueue_groups(st_ctx* c, const st::FusedParams& fp, size_t first,
                          const std::vector<size_t>& groups) {
   const size_t nj = groups.back() - first;
   ST_CUDA(st::launch_reset_aux((JobAux*)c->d_aux.p, (int)nj, c->stream), "reset aux");
-  if (c->cache_cells > 0) {
-    ST_CUDA(cudaMemsetAsync(c->c_cells.p, 0xFF, (size_t)c->cache_cells * sizeof(st::CellSlot), c->stream), "cell reset");
-  }
+  if (c->cache_bins > 0)
+    ST_CUDA(cudaMemsetAsync(c->z_bins.p, 0, (size_t)c->cache_bins * 4, c->stream), "z bin reset");
   ST_CUDA(cudaMemsetAsync(c->d_err.p, 0, 16, c->stream), "reset errors");
   ST_CUDA(cudaEventRecord(c->ev[0], c->stream), "event");
   for (size_t g = 0; g + 1 < groups.size(); ++g) {
@@ -839,7 +863,7 @@ st_status launch_range(st_ctx* c, size_t first, size_t last, bool want_export, i
   }
   const size_t n_groups = groups.size() - 1;
   c->launches += (nj > 0 ? 1 : 0) +
-                 (int32_t)n_groups * ((c->cache_blocks > 0 ? (c->cache_any_flagged ? 5 : 4) : 0) +
+                 (int32_t)n_groups * ((c->cache_blocks > 0 ? (c->cache_any_flagged ? 6 : 4) : 0) +
                                       (nj > 0 ? 4 : 0) + (c->cache_grid > 0 ? 1 : 0));
   c->pending = true;
   c->pend_first = first;
@@ -1051,7 +1075,7 @@ st_status st_ctx_destroy(st_ctx* c) {
   DevBuf* bufs[] = {&c->track_arena, &c->pxy, &c->pdz2, &c->pv, &c->pkey,
                     &c->d_jobs, &c->d_aux, &c->d_hists, &c->d_items, &c->d_blk,
                     &c->d_counter, &c->d_err, &c->d_blk_count, &c->d_blk_off, &c->d_blk_job, &c->c_cells,
-                    &c->pz, &c->u_next, &c->u_done, &c->u_table,
+                    &c->pz, &c->z_bins, &c->z_wins, &c->u_next, &c->u_done, &c->u_table,
                     &c->pool, &c->d_plan, &c->d_plan_misc, &c->g_keys, &c->g_lo, &c->g_hi,
                     &c->g_used, &c->g_count, &c->ex_buf, &c->ex_count, &c->h_counts,
                     &c->h_yfy, &c->h_edges};

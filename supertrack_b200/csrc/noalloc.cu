@@ -250,9 +250,6 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   NA_CUDA(cudaMemsetAsync(base + L.err, 0, 16, st_));
   NA_CUDA(cudaMemsetAsync(base + L.units, 0, 8, st_));
   NA_CUDA(cudaMemsetAsync(base + L.units + 8, 0xFF, 4, st_));
-  if (D.flagged) {
-    NA_CUDA(cudaMemsetAsync(base + L.cells, 0xFF, (size_t)kNaCellCap * sizeof(st::CellSlot), st_));
-  }
 
   st::PrepareParams pp;
   std::memset(&pp, 0, sizeof(pp));
@@ -264,6 +261,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   pp.blk_offset = (int64_t*)(base + L.blk_off);
   pp.cells = (st::CellSlot*)(base + L.cells);
   pp.blk_base = 0;
+  pp.any_flags = (int32_t*)(base + L.counter + 8);
   pp.PZ = (double*)(base + L.pz);
   pp.PXY = (double2*)(base + L.pxy);
 

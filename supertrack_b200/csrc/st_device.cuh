@@ -3,8 +3,8 @@
 // HBM layout of one batch:
 //   * input tracks: SoA float64 x, y, z, edep per job (caller memory or the context's arena);
 //   * prepared arena (written once per job, read once per oversample): for every job its kept
-//     deposits (those that can lie inside the voxel for some shift; in source order, or grouped
-//     by cell inside each prepare block) as a padded run of warp tiles of kWarpTile deposits.
+//     deposits (those that can lie inside the voxel for some shift; in source order, grouped by
+//     cell inside each prepare block, or ordered by z layer) as a padded run of warp tiles of kWarpTile deposits.
 //     Lane l of a warp tile owns the kDepPerLane consecutive deposits 4l..4l+3 of the tile,
 //     stored "pair-blocked" (prep_slot in vcs_kernels.cu): the pair 4l, 4l+1 at tile slots
 //     2l, 2l+1 and the pair 4l+2, 4l+3 at 64+2l, 64+2l+1, so a warp reads one pair per lane with
@@ -60,6 +60,15 @@ struct JobDev {
   int64_t cell_off;
   double cell_size;
   double inv_cell;    // RN(1 / cell_size)
+  // layer windows (see k_prep_write): with `layers` the job may be ordered by z layer; its n_bins bins of
+  // 2^bin_shift lattice layers are counted at [bin_off, bin_off + n_bins) of the bin arena, its
+  // windows listed from win_off of the window arena
+  int64_t bin_off;
+  int64_t win_off;
+  int32_t layers;
+  int32_t n_bins;
+  int32_t bin_shift;
+  int32_t reserved;
   // FP32 geometry variant: HL', gSO, d, RN(1/d) and r^2 rounded to float (1/d in float)
   float f_HL;
   float f_gSO;
@@ -75,19 +84,33 @@ struct JobDev {
 // of it; the flag travels in bit 63 of its PKEY word (keys are below 2^63).
 constexpr unsigned long long kBoundaryBit = 1ull << 63;
 
+// How a job's oversamples are cut into windows that empty the sphere table (JobAux::windowed):
+// not at all, windows of the source order with boundary flags, or windows of whole z layers.
+constexpr int kWinNone = 0;
+constexpr int kWinFlags = 1;
+constexpr int kWinLayers = 2;
+constexpr int kMaxBins = 4096;                        // z bins of a layered job
+constexpr unsigned long long kWinContinues = 1ull << 63;  // window list: the bin began earlier
+// Most entries of a job's window list: two consecutive windows hold more than one window's
+// deposits, a bin larger than a window ends with a short one, plus the closing entry.
+constexpr int64_t window_cap(int64_t n, int64_t win_deposits) { return 3 * (n / win_deposits) + 8; }
+
 // Per-job values produced on the device.
 struct JobAux {
   int32_t e_min;          // min ulp exponent over nonzero contributions
   int32_t e_max;          // max ulp exponent over nonzero contributions
   int32_t flags;          // kAuxNonzero | kAuxNonfinite
-  int32_t windowed;       // set by k_prep_scan: the job runs with window flags (JobDev::flagged
-                          // and more than PrepareParams::flag_min_kept kept deposits)
+  int32_t windowed;       // set by k_prep_scan: kWinNone, kWinFlags (JobDev::flagged and more
+                          // than PrepareParams::flag_min_kept kept deposits) or kWinLayers
   long long kept;              // deposits that can be inside the voxel for some shift
   unsigned long long hits;     // in-sphere deposits summed over all oversamples
   unsigned long long spheres;  // (oversample, sphere) pairs with at least one hit
   unsigned long long binned;   // of those, the ones that landed inside the histogram range
   unsigned long long inbox;    // deposit*oversamples inside the voxel after the shift
-  unsigned long long cells;    // occupied cells of the boundary-flag hash (windowed jobs)
+  unsigned long long cells;    // occupied cells: of the boundary-flag hash (kWinFlags), or of
+                               // each prepare block, summed (kWinLayers)
+  int32_t n_win;               // windows of a layered job
+  int32_t reserved;
 };
 constexpr int kAuxNonzero = 1;
 constexpr int kAuxNonfinite = 2;
@@ -108,6 +131,8 @@ struct WorkItem {
   int32_t os_count;
   int32_t unit;       // -1: the CTA does every window of os_begin..+os_count; else a helper of
                       // shared unit `unit` (one oversample of a large job, split into chunks)
+  int32_t win_begin;  // layered jobs: the windows of each oversample that the item covers
+  int32_t win_end;
 };
 
 // One exported sphere: (oversample, key, lineal energy, hit deposits).
@@ -149,6 +174,7 @@ struct FusedParams {
   unsigned int* unit_done;    // chunks finished
   int* unit_table;            // spill table of the unit (-1 none yet, -2 being acquired)
   unsigned int* pool_bits;    // spill tables in use (one bit per table, gridDim.x tables)
+  const unsigned long long* wins;  // window lists of layered jobs (first kept deposit of each)
   int32_t chunk_windows;      // windows per chunk
   int32_t fp32;               // 1: FP32 geometry variant (float records, float x/y geometry)
 };
@@ -176,6 +202,10 @@ struct PrepareParams {
   int32_t* blk_count;         // kept deposits per prepare block
   int64_t* blk_offset;        // first kept index of each prepare block inside its job
   CellSlot* cells;            // cell arena (flagged jobs)
+  uint32_t* bins;             // z bins of layered jobs: kept deposits, then first free place
+  unsigned long long* wins;   // window lists of layered jobs
+  int32_t win_tiles;          // warp tiles of a layer window (twice that on dense tracks)
+  int32_t* any_flags;         // set when a job of the launch runs with window boundary flags
   double* PZ;                 // z after the z-origin shift (flagged jobs only)
   double2* PXY;               // {x, y} per slot; FP32 variant: float2 {x, y} at the slot's index
   double* PDZ2;               // FP32 variant: float dz^2 at the slot's float index
@@ -196,6 +226,7 @@ struct JobPlan {
   int32_t bucket;
   int32_t unit_base;   // -1: private items
   int32_t blk_os;      // oversamples per private item, or helpers per unit
+  int32_t blk_win;     // layered jobs: windows per item (0: not layered)
 };
 struct PlanParams {
   const JobDev* jobs;

@@ -93,7 +93,14 @@ __device__ __forceinline__ int64_t prep_slot(const JobDev& J, int64_t k) {
 // coarse windows of kCoarseTiles warp tiles per warp; others with kWinTiles. Its cells record
 // windows of kWindow deposits, a coarse window is two of them.
 __device__ __forceinline__ bool coarse_windows(const JobDev& J, const JobAux& A) {
-  return A.windowed && (J.cell_nbr8 ? 4 : 2) * (long long)A.cells < A.kept;
+  return A.windowed == kWinFlags && (J.cell_nbr8 ? 4 : 2) * (long long)A.cells < A.kept;
+}
+
+// z bin of a kept deposit (z after the z-origin shift): its lattice layer k_z, clamped to the
+// lattice (k_z can round to -1 or N on the voxel's faces), over 2^bin_shift.
+__device__ __forceinline__ int z_bin(const JobDev& J, double z1) {
+  const int k = (int)lattice_index(st_dsub(z1, J.gSO), J.d, J.inv_d);
+  return min(max(k, 0), (int)J.N - 1) >> J.bin_shift;
 }
 
 __device__ __forceinline__ bool keep_deposit(const JobDev& J, double x, double y, double z) {
@@ -254,7 +261,17 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_count(PrepareParams p)
   for (int s = threadIdx.x; s < kPrepSlotsPerBlock; s += kPrepThreads) {
     const int64_t i = i0 + s;
     if (i >= J.n) continue;
-    kept += keep_deposit(J, J.x[i], J.y[i], J.z[i]) ? 1 : 0;
+    const double z = J.z[i];
+    const bool keep = keep_deposit(J, J.x[i], J.y[i], z);
+    kept += keep ? 1 : 0;
+    if (J.layers) {
+      // neighbouring deposits lie in few layers: one addition per layer and warp (one per deposit
+      // met on the same words: 7.9 ms instead of about 1.6 for 32e6 deposits of 10 nm ion tracks)
+      const int bin = keep ? z_bin(J, st_dadd(z, J.zsh)) : -1;
+      const unsigned same = __match_any_sync(__activemask(), bin);
+      if (keep && (int)(threadIdx.x & 31) == __ffs(same) - 1)
+        atomicAdd(&p.bins[J.bin_off + bin], (unsigned)__popc(same));
+    }
     const double v = __ddiv_rn(J.edep[i], J.denom);
     if (!isfinite(v)) {
       flags |= kAuxNonfinite;
@@ -303,6 +320,28 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_count(PrepareParams p)
   }
 }
 
+// Empties the cell hash of every job that runs with window boundary flags (all-ones is the empty
+// slot); any number of CTAs.
+__global__ void __launch_bounds__(kPrepThreads) k_prep_cells(PrepareParams p) {
+  if (!*p.any_flags) return;
+  __shared__ int s_jobs[kPrepThreads];
+  __shared__ int s_n;
+  for (int base = 0; base < p.n_jobs; base += kPrepThreads) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const int j = base + threadIdx.x;
+    if (j < p.n_jobs && p.aux[j].windowed == kWinFlags) s_jobs[atomicAdd(&s_n, 1)] = j;
+    __syncthreads();
+    for (int q = 0; q < s_n; ++q) {
+      const JobDev& J = p.jobs[s_jobs[q]];
+      uint4* slots = reinterpret_cast<uint4*>(p.cells + J.cell_off);
+      for (uint32_t i = blockIdx.x * kPrepThreads + threadIdx.x; i < J.cell_cap; i += gridDim.x * kPrepThreads)
+        slots[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    }
+    __syncthreads();
+  }
+}
+
 // One CTA per job: exclusive scan of the job's block counts.
 __global__ void __launch_bounds__(1024) k_prep_scan(PrepareParams p) {
   const int j = blockIdx.x;
@@ -339,9 +378,58 @@ __global__ void __launch_bounds__(1024) k_prep_scan(PrepareParams p) {
     if (threadIdx.x == 0) s_carry += s_warp[31];
     __syncthreads();
   }
+  const long long kept = s_carry;
+  const bool many = kept > p.flag_min_kept;
+  int mode = p.jobs[j].flagged && many ? kWinFlags : kWinNone;
+  if (p.jobs[j].layers && many) {
+    // the bin counts to first places, and the deposits that lie in bins larger than a window
+    uint32_t* bins = p.bins + p.jobs[j].bin_off;
+    const int nb = p.jobs[j].n_bins;
+    constexpr int kPer = kMaxBins / 1024;
+    unsigned v[kPer], sum = 0, big = 0;
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      const int b = (int)threadIdx.x * kPer + t;
+      v[t] = b < nb ? bins[b] : 0;
+      sum += v[t];
+      big += v[t] > (unsigned)(2 * kWindow) ? v[t] : 0;
+    }
+    unsigned incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    __shared__ unsigned s_bin[32];
+    __shared__ unsigned long long s_big;
+    if (threadIdx.x == 0) s_big = 0;
+    if (lane == 31) s_bin[warp] = incl;
+    __syncthreads();
+    if (big) atomicAdd(&s_big, (unsigned long long)big);
+    unsigned base = incl - sum;
+    for (int w = 0; w < warp; ++w) base += s_bin[w];
+#pragma unroll
+    for (int t = 0; t < kPer; ++t) {
+      const int b = (int)threadIdx.x * kPer + t;
+      if (b < nb) bins[b] = base;
+      base += v[t];
+    }
+    __syncthreads();
+    // Layers unless more than a quarter of the deposits lie in bins of over two windows (a track
+    // across z): such bins empty into the spill log piece by piece, where windows along the track
+    // would leave few boundary spheres. On dense tracks (over 1,024 deposits per sphere diameter
+    // of track length) a window along the track is hardly longer than a sphere, and the spheres
+    // of a large bin fit the table. Fused time of 8 ion tracks, layers / flags: along z, 1e6
+    // deposits, 2 nm 7.3 / 12.1 ms; across z, 1e6, 2 nm (sparse) 13.2 / 9.6, 1e6, 10 nm (1,000
+    // per diameter) 5.5 / 5.4, 4e6, 10 nm (4,000) 9.4 / 13.5, 2e6, 20 nm (8,000) 3.5 / 7.6.
+    const JobDev& J = p.jobs[j];
+    const bool dense = (double)J.n * J.d > 1024.0 * 2.0 * J.HL;
+    if (mode == kWinNone || dense || 4 * s_big <= (unsigned long long)kept) mode = kWinLayers;
+  }
   if (threadIdx.x == 0) {
-    p.aux[j].kept = s_carry;
-    p.aux[j].windowed = p.jobs[j].flagged && s_carry > p.flag_min_kept;
+    p.aux[j].kept = kept;
+    p.aux[j].windowed = mode;
+    if (mode == kWinFlags) *p.any_flags = 1;
   }
 }
 
@@ -362,6 +450,21 @@ __device__ __forceinline__ unsigned cell_hash_bin(const JobDev& J, double x, dou
   return ((cx * 73856093u) ^ (cy * 19349663u) ^ (cz * 83492791u)) & (kCellHashBins - 1);
 }
 
+// Layered jobs (kWinLayers). z is not shifted by an oversample, so a deposit's lattice layer k_z is
+// the same in all of them, and a sphere never leaves its layer: deposits ordered by layer can be cut
+// into windows of whole layers that share no sphere, whatever the shift. Every sphere of such a
+// window is complete when the window ends and is binned from shared memory, none goes through the
+// spill log, and any range of windows is a work item of its own (a large job spreads over the CTAs
+// without meeting in a table in HBM). The order is a counting sort: k_prep_count counts the z bins
+// (lattice layers, or 2^k of them), k_prep_scan turns the counts into first places, and here each
+// cell group of a block claims consecutive places in its bin, so that deposits of one cell stay
+// together. The places a bin's groups get depend on the blocks' timing, the results do not (sums are
+// exact). k_prep_pad cuts the windows.
+// Measured against windows of the source order with boundary flags (per pass): 8 tracks of 4e6
+// deposits, 10 nm, 50 oversamples 38.7 -> 25.4 ms; 16 of 1e6, 2 nm 27.1 -> 24.9; the
+// single-precision mix 7.8 -> 7.0; one track of 300,007 deposits 327 -> 295 us. The uneven
+// 2,048-track batch stays at 29.0 ms: its jobs of large spheres are not windowed.
+//
 // Four blocks per SM (64 registers, a few bytes of spills): the stage is memory-bound, and the
 // fourth block's loads in flight are worth more than the spills cost.
 __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p) {
@@ -380,15 +483,18 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
   __shared__ unsigned s_first[kCellHashBins];
   __shared__ unsigned s_group[kPrepSlotsPerBlock];
   __shared__ unsigned s_part[kWarpsPerBlock];
+  __shared__ unsigned s_base[kPrepSlotsPerBlock];  // layered jobs: first place of each group
+  __shared__ unsigned short s_zbin[kPrepSlotsPerBlock];  // and its z bin
   int64_t run = p.blk_offset[b];  // kept index of the next kept deposit of this block
-  const bool sorted = p.sort == 2 || (p.sort == 1 && J.flagged);
+  const JobAux A = p.aux[j];
+  const bool layered = A.windowed == kWinLayers;
+  const bool sorted = p.sort == 2 || (p.sort == 1 && (J.flagged || layered));
   if (sorted) {
 #pragma unroll
     for (int t = 0; t < kHashPerThread; ++t) s_first[threadIdx.x * kHashPerThread + t] = ~0u;
 #pragma unroll
     for (int t = 0; t < kGroupsPerThread; ++t) s_group[threadIdx.x * kGroupsPerThread + t] = 0;
   }
-  const JobAux A = p.aux[j];
   const int E0 = choose_grid_exponent(A.e_min, A.e_max, J.n, A.flags & kAuxNonzero);
   unsigned created_cells = 0;  // cells this thread created (windowed jobs)
   // the loads of all rounds are issued before the block's one barrier, so each thread has all
@@ -423,7 +529,35 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
     }
   }
   __syncthreads();
-  if (sorted) {
+  if (layered) {
+    // Each group (named by its first deposit, which claims for it) takes consecutive places in
+    // its z bin; a deposit whose hash collided with a group of another bin claims its own.
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const unsigned own = r * kPrepThreads + threadIdx.x;
+      if (keep & (1u << r)) s_zbin[own] = (unsigned short)z_bin(J, z1[r]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      if (keep & (1u << r)) {
+        const unsigned own = r * kPrepThreads + threadIdx.x;
+        const unsigned first = s_first[slot_of[r]];
+        const unsigned g = s_zbin[first] == s_zbin[own] ? first : own;
+        slot_of[r] = (g << 16) | atomicAdd(&s_group[g], 1u);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const unsigned own = r * kPrepThreads + threadIdx.x;
+      if ((keep & (1u << r)) && (slot_of[r] >> 16) == own) {
+        s_base[own] = atomicAdd(&p.bins[J.bin_off + s_zbin[own]], s_group[own]);
+        ++created_cells;
+      }
+    }
+    __syncthreads();
+  } else if (sorted) {
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
       if (keep & (1u << r)) {
@@ -471,7 +605,8 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
     if (keep & (1u << r)) {
       // kept index: block order, or the position of the deposit's group and rank in sorted
       // blocks
-      const int64_t k = sorted ? p.blk_offset[b] + s_group[slot_of[r] >> 16] + (slot_of[r] & 0xFFFFu)
+      const int64_t k = layered ? (int64_t)s_base[slot_of[r] >> 16] + (slot_of[r] & 0xFFFFu)
+                        : sorted ? p.blk_offset[b] + s_group[slot_of[r] >> 16] + (slot_of[r] & 0xFFFFu)
                                : run + before + __popc(m[r] & ((1u << lane) - 1u));
       const double az = st_dsub(z1[r], J.gSO);
       const double kd = lattice_index(az, J.d, J.inv_d);
@@ -488,13 +623,13 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
       to_fixed(__ddiv_rn(e[r], J.denom), E0, &lo, &hi);
       p.PV[dst] = make_ulonglong2(lo, hi);
       p.PKEY[dst] = (uint64_t)(long long)kd * J.N2;
-      if (A.windowed) {
+      if (A.windowed == kWinFlags) {
         p.PZ[dst] = z1[r];
         ckey = cell_key(cell_of(x[r], y[r], z1[r], J.inv_cell), 0, 0, 0);
         cwin = (uint32_t)(k / kWindow);
       }
     }
-    if (A.windowed) {
+    if (A.windowed == kWinFlags) {
       // adjacent lanes hold adjacent source deposits, which on dense tracks share a cell and a
       // window: an insert equal to the previous lane's changes nothing and is skipped, which
       // spares the cell's slot most of its same-address atomics
@@ -517,11 +652,57 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
   }
 }
 
-// One block per job: padding slots [kept, kept rounded up to a warp tile).
+// Window list of a layered job, by one warp: from the first place k0 of a window, whose tile span
+// ends at `limit`, the window ends after the last bin that ends by then, or at `limit` when the
+// bin itself goes on (its next window is marked kWinContinues). bins[b] is the end of bin b.
+__device__ __forceinline__ void cut_windows(const PrepareParams& p, const JobDev& J, JobAux* aux,
+                                            const uint32_t* bins) {
+  const int lane = threadIdx.x;
+  unsigned long long* wins = p.wins + J.win_off;
+  const long long kept = aux->kept;
+  const long long tiles = 2 * (long long)aux->cells < kept ? 2 * p.win_tiles : p.win_tiles;
+  long long k0 = 0;
+  unsigned long long mark = 0;
+  int n = 0, b = 0;  // b: first bin that ends behind k0
+  while (k0 < kept) {
+    if (lane == 0) wins[n] = (unsigned long long)k0 | mark;
+    ++n;
+    const long long limit = (k0 / kWarpTile + tiles) * kWarpTile;
+    long long end = k0;  // end of the last bin that ends by `limit`
+    for (;; ) {
+      const long long e = b + lane < J.n_bins ? (long long)bins[b + lane] : LLONG_MAX;
+      const unsigned in = __ballot_sync(0xffffffffu, e <= limit);  // a prefix of the lanes
+      if (in == 0) break;
+      end = __shfl_sync(0xffffffffu, e, 31 - __clz(in));
+      b += __popc(in);
+      if (in != 0xffffffffu) break;
+    }
+    if (end > k0) {
+      k0 = end;
+      mark = 0;
+    } else {
+      k0 = limit;
+      mark = kWinContinues;
+    }
+  }
+  if (lane == 0) {
+    wins[n] = (unsigned long long)kept;
+    aux->n_win = n;
+  }
+}
+
+// One block per job: padding slots [kept, kept rounded up to a warp tile), and the window list of
+// a layered job.
 __global__ void __launch_bounds__(kWarpTile) k_prep_pad(PrepareParams p) {
   const int j = blockIdx.x;
   const JobDev J = p.jobs[j];
   const long long kept = p.aux[j].kept;
+  if (p.aux[j].windowed == kWinLayers) {
+    __shared__ uint32_t s_ends[kMaxBins];
+    for (int b = threadIdx.x; b < J.n_bins; b += kWarpTile) s_ends[b] = p.bins[J.bin_off + b];
+    __syncthreads();
+    if (threadIdx.x < 32) cut_windows(p, J, &p.aux[j], s_ends);
+  }
   if ((kept % kWarpTile) == 0) return;
   const long long k = kept + threadIdx.x;
   if (k >= (kept / kWarpTile + 1) * kWarpTile) return;
@@ -545,11 +726,12 @@ __global__ void __launch_bounds__(kWarpTile) k_prep_pad(PrepareParams p) {
 // so the fused kernel can bin it as soon as the window is done.
 // Eight blocks per SM (32 registers): the cell probes are L2 latency, which more warps hide.
 __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_flag(PrepareParams p) {
+  if (!*p.any_flags) return;
   const int64_t b = p.blk_base + blockIdx.x;
   const int j = prep_job(p, b);
   const JobDev J = p.jobs[j];
   const JobAux A = p.aux[j];
-  if (!A.windowed) return;
+  if (A.windowed != kWinFlags) return;
   const int shift = coarse_windows(J, A) ? 1 : 0;
   const int64_t k0 = p.blk_offset[b];
   const int cnt = p.blk_count[b];
@@ -1111,6 +1293,7 @@ __device__ __forceinline__ void log_reduce(const SmemTable<CAP>& T, CtaState& cs
 
 struct FusedJob {
   JobDev J;
+  const unsigned long long* wins;  // layered jobs: the window list, else null
   int E0;
   int win_tiles;    // warp tiles per warp in a window: kWinTiles, or kCoarseTiles
   int64_t n_wt;     // warp tiles of kept deposits
@@ -1125,8 +1308,10 @@ __host__ __device__ __forceinline__ int64_t chunk_tiles(int chunk_windows) {
 }
 
 // Superimposes oversample `os` of a job over warp tiles [wt_begin, wt_end) (whole windows):
-// shift, box test, lattice test, key, exact run / shared-memory reduction. For flagged jobs
-// every window ends by binning its complete spheres and moving boundary spheres to G; otherwise
+// shift, box test, lattice test, key, exact run / shared-memory reduction. For layered jobs the
+// range is one of windows of F.wins instead. For windowed jobs every window ends by binning its
+// complete spheres and moving boundary spheres to G (layered jobs have none, except the parts of a
+// bin larger than a window whose spheres fill the table); otherwise
 // spheres accumulate across windows and the shared table spills to G when it fills up.
 // F32: the FP32 geometry variant (x, y, shifts, lattice index and distance in float; z part of
 // the distance, keys and energies as in the FP64 form).
@@ -1134,7 +1319,7 @@ template <int CAP, int THREADS, bool F32>
 __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob& F,
                                             const SmemTable<CAP>& T, CtaState& cs,
                                             const Spill& G, const BinContext& B, int os,
-                                            int64_t wt_begin, int64_t wt_end,
+                                            int64_t begin, int64_t end,
                                             unsigned int& hits, unsigned int& inbox,
                                             unsigned int& spheres, unsigned int& binned) {
   constexpr int kWarps = THREADS / 32;
@@ -1153,18 +1338,35 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
   const bool log_mode = cs.log_mode != 0;
   const bool window_checks = CAP < 2 * kCtaTile && !J.flagged &&
                              (uint64_t)J.N * J.N2 > (uint64_t)P.flush_threshold;
-  int wi = 0;  // window index within this call
-  const int wtiles = F.win_tiles;
-  for (int64_t wt0 = wt_begin; wt0 < wt_end; wt0 += kWarps * wtiles) {
+  int wi = 0;  // emptied windows within this call
+  bool logged = false;  // part of the current layer bin is in the spill log
+  for (int64_t at = begin; at < end;) {
     const int slot = J.flagged ? wi % 3 : 0;
-    // a window is wtiles warp tiles per warp
+    // the window's warp tiles [w0, w1): win_tiles per warp from tile `at`, or window `at` of the
+    // list, which may begin and end inside a tile (clip0: its first deposit in tile w0, clip1:
+    // one past its last in tile w1 - 1)
+    int w0, w1, clip0 = 0, clip1 = kWarpTile;
+    bool more = false;  // the next window continues this one's last bin
+    if (F.wins) {
+      const unsigned long long a = __ldg(&F.wins[at]), b = __ldg(&F.wins[at + 1]);
+      const long long k0 = (long long)(a & ~kWinContinues), k1 = (long long)(b & ~kWinContinues);
+      more = (b & kWinContinues) != 0;
+      w0 = (int)(k0 / kWarpTile);
+      w1 = (int)((k1 + kWarpTile - 1) / kWarpTile);
+      clip0 = (int)(k0 % kWarpTile);
+      clip1 = (int)(k1 - (long long)(w1 - 1) * kWarpTile);
+      ++at;
+    } else {
+      w0 = (int)at;
+      at = at + kWarps * F.win_tiles < end ? at + kWarps * F.win_tiles : end;
+      w1 = (int)at;
+    }
 #pragma unroll 1
-    for (int tt = 0; tt < wtiles; ++tt) {
-      const int64_t w = wt0 + tt * kWarps + warp;
-      if (w < wt_end) {
+    for (int w = w0 + warp; w < w1; w += kWarps) {
+      {
         // pair-blocked tile (prep_slot): this lane's deposits p = 0, 1 are the slots tb, tb + 1
         // and p = 2, 3 the slots tb + 64, tb + 65
-        const int64_t tb = J.prep_off + w * kWarpTile + 2 * lane;
+        const int64_t tb = J.prep_off + (int64_t)w * kWarpTile + 2 * lane;
         uint32_t kxv[kDepPerLane], kyv[kDepPerLane];
         unsigned hitmask = 0, boxmask = 0;
         if constexpr (F32) {
@@ -1247,6 +1449,13 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
           }
         }
         }
+        if (F.wins) {  // lane's deposits 4 * lane + 0..3 of the tile that the window holds
+          unsigned in = 0xFu;
+          if (w == w0) in &= 0xFu << min(max(clip0 - 4 * lane, 0), 4);
+          if (w == w1 - 1) in &= (1u << min(max(clip1 - 4 * lane, 0), 4)) - 1u;
+          hitmask &= in;
+          boxmask &= in;
+        }
         hits += __popc(hitmask);
         inbox += __popc(boxmask);
         // runs of equal keys inside the lane's consecutive deposits are summed in registers
@@ -1287,7 +1496,12 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
       // the others (or all, if the window overflowed) go to the spill table
       __syncthreads();
       const int cnt = cs.tc[slot];
-      const bool all_out = cs.ovf[slot] != 0;
+      if (more && cnt <= CAP / 2) {  // a bin larger than a window, and room for more spheres
+        __syncthreads();  // (every thread has read the count)
+        continue;
+      }
+      const bool all_out = cs.ovf[slot] != 0 || more || logged;
+      logged = more;
       if (tid == 0) {  // the next window's slot: last read two windows ago
         cs.tc[(wi + 1) % 3] = 0;
         cs.ovf[(wi + 1) % 3] = 0;
@@ -1313,7 +1527,7 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
       // the table and its boundary bits are clear again once every thread is past this point
       sent = __syncthreads_or(sent);
       if (sent && tid == 0) cs.spilled = 1;
-    } else if (window_checks && wt0 + kWarps * wtiles < wt_end) {
+    } else if (window_checks && at < end) {
       __syncthreads();
       if (cs.tc[0] > P.flush_threshold) {
         if (log_mode) flush_to_log<CAP, THREADS>(T, cs.tc[0], &cs, P, G);
@@ -1377,7 +1591,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     if (A.flags & kAuxNonfinite) continue;  // rejected job: contributes nothing, host reports it
     FusedJob F;
     F.J = P.jobs[W.job];
-    F.J.flagged = A.windowed;  // window flags were computed only for these jobs
+    F.J.flagged = A.windowed;  // window flags and lists were computed only for these jobs
+    F.wins = A.windowed == kWinLayers ? P.wins + F.J.win_off : nullptr;
     F.win_tiles = coarse_windows(F.J, A) ? kCoarseTiles : kWinTiles;
     F.E0 = choose_grid_exponent(A.e_min, A.e_max, F.J.n, A.flags & kAuxNonzero);
     F.n_wt = (A.kept + kWarpTile - 1) / kWarpTile;
@@ -1433,6 +1648,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
         t = private_table;
         wb = 0;
         we = F.n_wt;
+        if (F.wins) {
+          // whole bins: a window that continues a bin belongs to the item that began it
+          wb = W.win_begin;
+          we = W.win_end;
+          while (wb < A.n_win && (F.wins[wb] & kWinContinues)) ++wb;
+          while (we < A.n_win && (F.wins[we] & kWinContinues)) ++we;
+        }
       } else {
         if (tid == 0) {
           const unsigned c = atomicAdd(&P.unit_next[W.unit], 1u);
@@ -1573,6 +1795,14 @@ __device__ __forceinline__ int cost_bucket(long long cost) {
   return kPlanBuckets - 1 - l;  // larger cost -> smaller bucket -> earlier
 }
 
+// Work of one item: item_cost, less in a batch too small to give every CTA several items.
+__device__ __forceinline__ long long plan_item_cost(const PlanParams& q) {
+  const long long share = (long long)(*q.total_units / ((unsigned long long)q.grid * 8));
+  const long long lo = 4096;
+  const long long ic = share < lo ? lo : share;
+  return ic < q.item_cost ? ic : q.item_cost;
+}
+
 __global__ void k_plan_size(PlanParams q) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= q.n_jobs) return;
@@ -1583,11 +1813,34 @@ __global__ void k_plan_size(PlanParams q) {
   pl.bucket = kPlanBuckets - 1;
   pl.unit_base = -1;
   pl.blk_os = 1;
+  pl.blk_win = 0;
   if (kept > 0 && nos > 0 && !(q.aux[j].flags & kAuxNonfinite)) {
     const long long chunk = chunk_tiles(q.chunk_windows) * kWarpTile;
     const long long share =
         q.share_divisor > 0 ? (long long)(*q.total_units / ((unsigned long long)q.share_divisor * q.grid)) : 0;
-    if (q.share_divisor > 0 && kept > (long long)q.min_chunks * chunk && kept > share) {
+    if (q.aux[j].windowed == kWinLayers) {
+      // any range of windows is complete on its own: about item_cost of work per item, as whole
+      // oversamples or as parts of one
+      const long long n_win = q.aux[j].n_win;
+      const long long ic = plan_item_cost(q);
+      if (kept > ic && n_win > 1) {
+        long long parts = (kept + ic - 1) / ic;
+        parts = parts < q.max_helpers ? parts : q.max_helpers;
+        parts = parts < n_win ? parts : n_win;
+        const long long per = (n_win + parts - 1) / parts;
+        pl.blk_win = (int)per;
+        pl.blk_os = 1;
+        pl.items = (int)(nos * ((n_win + per - 1) / per));
+        pl.bucket = cost_bucket(kept / parts);
+      } else {
+        long long b = ic / kept;
+        b = b < 1 ? 1 : (b > nos ? nos : b);
+        pl.blk_win = (int)n_win;
+        pl.blk_os = (int)b;
+        pl.items = (int)((nos + b - 1) / b);
+        pl.bucket = cost_bucket(kept * b);
+      }
+    } else if (q.share_divisor > 0 && kept > (long long)q.min_chunks * chunk && kept > share) {
       const long long chunks = (kept + chunk - 1) / chunk;
       const int helpers = (int)(chunks < q.max_helpers ? chunks : q.max_helpers);
       pl.blk_os = helpers;
@@ -1632,7 +1885,18 @@ __global__ void __launch_bounds__(128) k_plan_write(PlanParams q) {
     if (pos >= q.item_cap) break;
     WorkItem w;
     w.job = j;
-    if (pl.unit_base >= 0) {
+    w.win_begin = 0;
+    w.win_end = 0;
+    if (pl.blk_win > 0) {
+      const int n_win = q.aux[j].n_win;
+      const int parts = (n_win + pl.blk_win - 1) / pl.blk_win;
+      const int o = k / parts, part = k % parts;
+      w.os_begin = o * pl.blk_os;
+      w.os_count = (w.os_begin + pl.blk_os <= nos) ? pl.blk_os : nos - w.os_begin;
+      w.unit = -1;
+      w.win_begin = part * pl.blk_win;
+      w.win_end = min(w.win_begin + pl.blk_win, n_win);
+    } else if (pl.unit_base >= 0) {
       const int u = k / pl.blk_os;
       w.os_begin = u;
       w.os_count = 1;
@@ -1663,6 +1927,8 @@ __global__ void k_reset_aux(JobAux* aux, int n) {
   a.binned = 0;
   a.inbox = 0;
   a.cells = 0;
+  a.n_win = 0;
+  a.reserved = 0;
   aux[j] = a;
 }
 
@@ -1754,6 +2020,10 @@ constexpr int kFusedThreads = 1024;
 constexpr int kSmallHistBins = 600;
 constexpr int kBigHistBins = 4096;
 
+bool fused_big_table(int max_nbins, int table_slots) {
+  return max_nbins <= kSmallHistBins && table_slots != 4096;
+}
+
 size_t fused_smem_bytes(int cap, int hist_bins) {
   return (size_t)cap * 26 + (size_t)cap / 8 + (size_t)hist_bins * 28 + 8;
 }
@@ -1763,6 +2033,7 @@ cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_fl
   if (n_blocks <= 0) return cudaSuccess;
   k_prep_count<<<(unsigned)n_blocks, kPrepThreads, 0, s>>>(p);
   k_prep_scan<<<p.n_jobs, 1024, 0, s>>>(p);
+  if (any_flagged) k_prep_cells<<<592, kPrepThreads, 0, s>>>(p);
   k_prep_write<<<(unsigned)n_blocks, kPrepThreads, 0, s>>>(p);
   k_prep_pad<<<p.n_jobs, kWarpTile, 0, s>>>(p);
   if (any_flagged) k_prep_flag<<<(unsigned)n_blocks, kPrepThreads, 0, s>>>(p);
@@ -1801,7 +2072,7 @@ static void launch_fused_form(const FusedParams& p, int grid, bool big_table, cu
 // geometry form.
 cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s) {
   if (grid <= 0) return cudaSuccess;
-  const bool big_table = max_nbins <= kSmallHistBins && table_slots != 4096;
+  const bool big_table = fused_big_table(max_nbins, table_slots);
   if (big_table) {
     p.smem_hist_bins = kSmallHistBins;
     p.flush_threshold = 8192 - 4096 - 8192 / 4;  // unused: no window checks on this table
