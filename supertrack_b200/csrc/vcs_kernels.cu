@@ -891,6 +891,8 @@ struct CtaState {
   int edges_hist;   // histogram whose edges are in shared memory (-1: none)
   int log_mode;     // private item: table overflows, flushes and window-end spills go to the log
   int logn;         // records in the spill log of this oversample
+  int table;        // spill table that the CTA holds for its private items (-1: none)
+  long long hist_work;  // deposit*oversamples in the shared-memory histogram
 };
 
 // Spill table of the current item: the CTA's table restricted to a power-of-two prefix sized
@@ -1547,6 +1549,33 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
 // oversamples of a small or medium job, one CTA) or helpers of a shared unit (one oversample of
 // a large job, whose window chunks are claimed dynamically by every helper that arrives).
 // ---------------------------------------------------------------------------------------------
+// Adds the shared-memory copies of a histogram to HBM and clears them (all threads of the CTA).
+template <int THREADS>
+__device__ __forceinline__ void flush_histogram(const HistDev& H, int HB, const double* sedges,
+                                                unsigned int* hcount, unsigned long long* hylo,
+                                                unsigned long long* hyhi) {
+  const int copies = min(kHistCopies, HB / H.nbins);
+  for (int b = threadIdx.x; b < H.nbins; b += THREADS) {
+    unsigned cnt = 0;
+    for (int c = 0; c < copies; ++c) cnt += hcount[c * H.nbins + b];
+    if (!cnt) continue;  // nothing in the bin's sums either
+    const uint64_t eb = (uint64_t)__double_as_longlong(sedges[b]);
+    const bool exact = (int64_t)eb > 0 && (eb >> 52) != 0;  // as in bin_sphere
+    uint64_t lo = 0, hi = 0;
+    double ys = 0.0;
+    for (int c = 0; c < copies; ++c) {
+      const int i = c * H.nbins + b;
+      if (exact) add128(lo, hi, hylo[i], hyhi[i]);
+      else ys += __longlong_as_double((long long)hylo[i]);
+      hcount[i] = 0;
+      hylo[i] = 0;
+      hyhi[i] = 0;
+    }
+    atomicAdd(&H.counts[b], (unsigned long long)cnt);
+    atomicAdd(&H.yfy[b], exact ? from_fixed(lo, hi, (int)(eb >> 52) - 1075) : ys);
+  }
+}
+
 template <int CAP, int THREADS, bool F32>
 __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
   static_assert(CAP <= 65536, "used-slot list stores 16-bit slot indices");
@@ -1575,6 +1604,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     cs.log_mode = 0;
     cs.logn = 0;
     cs.edges_hist = -1;
+    cs.table = -1;
+    cs.hist_work = 0;
   }
   __syncthreads();
 
@@ -1583,6 +1614,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     __syncthreads();
     const int it = cs.item;
     const int cached_hist = cs.edges_hist;
+    const long long hist_work = cs.hist_work;
     __syncthreads();
     if (it >= *P.n_items) break;
 
@@ -1599,14 +1631,27 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     const HistDev H = P.hists[F.J.hist];
     const bool smem_hist = H.nbins <= HB;
 
-    // histogram edges into shared memory (kept while consecutive items use the same histogram)
-    if (smem_hist && cached_hist != F.J.hist) {
+    // the histogram in shared memory: edges and sums stay while consecutive items use the same
+    // one (each item fills a bin by at most its own deposit*oversamples: they are added to HBM
+    // before the 32-bit counts could wrap). 64 short tracks on one 3,000-bin spectrum: fused
+    // 0.108 ms with a flush per item, 0.089 ms without.
+    const long long work = A.kept * W.os_count;
+    const bool full = hist_work + work > (1ll << 31);
+    if (smem_hist && (cached_hist != F.J.hist || full)) {
+      if (cached_hist >= 0) {
+        flush_histogram<THREADS>(P.hists[cached_hist], HB, sedges, hcount, hylo, hyhi);
+        __syncthreads();
+      }
       for (int i = tid; i <= H.nbins; i += THREADS) sedges[i] = H.edges[i];
       __syncthreads();
-      if (tid == 0) cs.edges_hist = F.J.hist;
+      if (tid == 0) {
+        cs.edges_hist = F.J.hist;
+        cs.hist_work = 0;
+      }
     }
 
     if (tid == 0) {
+      cs.hist_work += work;
       sB.edges = smem_hist ? sedges : H.edges;
       sB.gcounts = H.counts;
       sB.gyfy = H.yfy;
@@ -1632,13 +1677,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     const bool shared = W.unit >= 0;
     const int64_t wpc = chunk_tiles(P.chunk_windows);  // warp tiles per chunk
     const int64_t n_chunks = (F.n_wt + wpc - 1) / wpc;
-    int private_table = -1;
-    if (!shared) {
-      if (tid == 0) s_bcast[0] = pool_acquire(P.pool_bits, gridDim.x, P.error_flags);
-      __syncthreads();
-      private_table = s_bcast[0];
-      __syncthreads();
+    // A private item's spill table stays with the CTA for its next private items; it goes back to
+    // the pool before the CTA joins a shared unit, so that a CTA holds at most one.
+    if (tid == 0) {
+      if (!shared && cs.table < 0) {
+        cs.table = pool_acquire(P.pool_bits, gridDim.x, P.error_flags);
+      } else if (shared && cs.table >= 0) {
+        __threadfence();
+        pool_release(P.pool_bits, cs.table);
+        cs.table = -1;
+      }
     }
+    __syncthreads();
+    const int private_table = cs.table;
     for (int seg = 0;; ++seg) {
       int os, t;
       int64_t wb, we;
@@ -1725,36 +1776,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
       }
       __syncthreads();
     }
-    if (private_table >= 0) {
-      __threadfence();
-      __syncthreads();
-      if (tid == 0) pool_release(P.pool_bits, private_table);
-    }
-
-    // ---- per-item flush of the shared-memory histogram and the job statistics
-    if (smem_hist) {
-      const int copies = B.copies;
-      for (int b = tid; b < H.nbins; b += THREADS) {
-        const uint64_t eb = (uint64_t)__double_as_longlong(sedges[b]);
-        const bool exact = (int64_t)eb > 0 && (eb >> 52) != 0;  // as in bin_sphere
-        unsigned cnt = 0;
-        uint64_t lo = 0, hi = 0;
-        double ys = 0.0;
-        for (int c = 0; c < copies; ++c) {
-          const int i = c * H.nbins + b;
-          cnt += hcount[i];
-          if (exact) add128(lo, hi, hylo[i], hyhi[i]);
-          else ys += __longlong_as_double((long long)hylo[i]);
-          hcount[i] = 0;
-          hylo[i] = 0;
-          hyhi[i] = 0;
-        }
-        if (cnt) {
-          atomicAdd(&H.counts[b], (unsigned long long)cnt);
-          atomicAdd(&H.yfy[b], exact ? from_fixed(lo, hi, (int)(eb >> 52) - 1075) : ys);
-        }
-      }
-    }
     unsigned long long w_hits = hits, w_spheres = spheres, w_binned = binned, w_inbox = inbox;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1771,6 +1792,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     }
     __syncthreads();
   }
+  if (cs.edges_hist >= 0)
+    flush_histogram<THREADS>(P.hists[cs.edges_hist], HB, sedges, hcount, hylo, hyhi);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1795,10 +1818,15 @@ __device__ __forceinline__ int cost_bucket(long long cost) {
   return kPlanBuckets - 1 - l;  // larger cost -> smaller bucket -> earlier
 }
 
-// Work of one item: item_cost, less in a batch too small to give every CTA several items.
+// Work of one item: item_cost, or an eighth of a CTA's share of a batch too small for that, down
+// to 2,048 deposit*oversamples (half of a warp tile per warp; smaller items cost as much). With
+// items of item_cost a single proton track of 100 oversamples ran on 3 of the 148 CTAs: fused
+// 0.40 ms, against 0.062 ms split; a track of 10 oversamples, one at a time, 84 -> 25 us. A half
+// instead of an eighth of the share made groups of uneven tracks wait for their largest items
+// (6.2 against 5.6 ms for 256 host tracks in groups).
 __device__ __forceinline__ long long plan_item_cost(const PlanParams& q) {
   const long long share = (long long)(*q.total_units / ((unsigned long long)q.grid * 8));
-  const long long lo = 4096;
+  const long long lo = 2048;
   const long long ic = share < lo ? lo : share;
   return ic < q.item_cost ? ic : q.item_cost;
 }
@@ -1849,7 +1877,7 @@ __global__ void k_plan_size(PlanParams q) {
       pl.bucket = cost_bucket(kept);
     } else {
       const long long pad = ((kept + kWarpTile - 1) / kWarpTile) * kWarpTile;
-      long long b = q.item_cost / pad;
+      long long b = plan_item_cost(q) / pad;
       b = b < 1 ? 1 : (b > nos ? nos : b);
       pl.blk_os = (int)b;
       pl.items = (int)((nos + b - 1) / b);
