@@ -141,7 +141,7 @@ struct st_ctx {
   std::vector<JobHost> jobs;
 
   DevBuf track_arena;
-  DevBuf pxy, pdz2, pv, pkey;
+  DevBuf pg, pgz, pxy, pdz2, pv, pkey;
   DevBuf d_jobs, d_aux, d_hists, d_items, d_blk, d_counter, d_err, d_blk_count, d_blk_off, d_blk_job;
   DevBuf c_cells, pz;               // cell arena and shifted z of flagged jobs
   DevBuf z_bins, z_wins;            // z bins and window lists of layered jobs
@@ -312,9 +312,11 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
       arena_total += J.track.n;
     }
   }
-  ST_CUDA(ensure(c->pxy, prep_total * 16), "prepared arena");
-
-  ST_CUDA(ensure(c->pdz2, prep_total * 8), "prepared arena");
+  const int64_t exact_total = c->precision == 32 ? 0 : prep_total;  // FP64 records
+  ST_CUDA(ensure(c->pg, prep_total * 8), "prepared arena");
+  ST_CUDA(ensure(c->pgz, prep_total * 4), "prepared arena");
+  ST_CUDA(ensure(c->pxy, exact_total * 16), "prepared arena");
+  ST_CUDA(ensure(c->pdz2, exact_total * 8), "prepared arena");
   ST_CUDA(ensure(c->pv, prep_total * 16), "prepared arena");
   ST_CUDA(ensure(c->pkey, prep_total * 8), "prepared arena");
   ST_CUDA(ensure(c->track_arena, (size_t)arena_total * 32), "track arena");
@@ -388,6 +390,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
     D.f_d = (float)J.g.sphereDiameter;
     D.f_inv_d = 1.0f / D.f_d;
     D.f_r2 = (float)D.r2;
+    st::set_integer_geometry(&D);
     if (D.flagged) {
       D.cell_cap = next_pow2((uint64_t)2 * (uint64_t)J.track.n);
       D.cell_off = cells_total;
@@ -533,8 +536,9 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   pp.win_tiles = win_tiles;
   pp.any_flags = (int32_t*)((char*)c->d_counter.p + 8);
   pp.PZ = (double*)c->pz.p;
+  pp.PG = (int2*)c->pg.p;
+  pp.PGZ = (float*)c->pgz.p;
   pp.PXY = (double2*)c->pxy.p;
-
   pp.PDZ2 = (double*)c->pdz2.p;
   pp.PV = (ulonglong2*)c->pv.p;
   pp.PKEY = (unsigned long long*)c->pkey.p;
@@ -550,6 +554,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   fp.n_items = (const int*)((char*)c->d_plan_misc.p + 8);
   fp.flush_threshold = 1024;
   fp.work_counter = (unsigned int*)c->d_counter.p;
+  fp.PG = pp.PG; fp.PGZ = pp.PGZ;
   fp.PXY = pp.PXY; fp.PDZ2 = pp.PDZ2;
   fp.PV = pp.PV; fp.PKEY = pp.PKEY;
   fp.gkeys = (uint64_t*)c->g_keys.p;
@@ -1072,7 +1077,7 @@ st_status st_ctx_destroy(st_ctx* c) {
   if (!c) return ST_ERR_INVALID_ARGUMENT;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  DevBuf* bufs[] = {&c->track_arena, &c->pxy, &c->pdz2, &c->pv, &c->pkey,
+  DevBuf* bufs[] = {&c->track_arena, &c->pg, &c->pgz, &c->pxy, &c->pdz2, &c->pv, &c->pkey,
                     &c->d_jobs, &c->d_aux, &c->d_hists, &c->d_items, &c->d_blk,
                     &c->d_counter, &c->d_err, &c->d_blk_count, &c->d_blk_off, &c->d_blk_job, &c->c_cells,
                     &c->pz, &c->z_bins, &c->z_wins, &c->u_next, &c->u_done, &c->u_table,

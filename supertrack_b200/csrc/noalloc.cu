@@ -57,7 +57,7 @@ constexpr size_t al(size_t v) { return (v + 255) / 256 * 256; }
 // Byte offsets of every region inside the scratch array.
 struct Layout {
   size_t jobs, aux, hists, blk_prefix, blk_count, blk_off;
-  size_t pxy, pdz2, pv, pkey, pz;
+  size_t pg, pgz, pxy, pdz2, pv, pkey, pz;
   size_t cells;
   size_t gkeys, glo, ghi, gused, gcount, pool;
   size_t items, plan, plan_misc, counter, err, edges, units;
@@ -73,8 +73,9 @@ constexpr Layout make_layout() {
   L.blk_prefix = o; o += al(2 * 8);
   L.blk_count = o;  o += al(kNaBlocks * 4);
   L.blk_off = o;    o += al(kNaBlocks * 8);
+  L.pg = o;         o += al(kNaMaxDeposits * 8);
+  L.pgz = o;        o += al(kNaMaxDeposits * 4);
   L.pxy = o;        o += al(kNaMaxDeposits * 16);
-
   L.pdz2 = o;       o += al(kNaMaxDeposits * 8);
   L.pv = o;         o += al(kNaMaxDeposits * 16);
   L.pkey = o;       o += al(kNaMaxDeposits * 8);
@@ -205,6 +206,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   D.cell_nbr8 = (D.flagged && per_d * desc->n_oversamples <= (double)st::kFlagCellsLimit) ? 1 : 0;
   D.cell_size = (D.cell_nbr8 ? 2.0 : 1.0) * g.sphereDiameter * (1.0 + 0x1p-10);
   D.inv_cell = 1.0 / D.cell_size;
+  st::set_integer_geometry(&D);
 
   st::JobAux A;
   std::memset(&A, 0, sizeof(A));
@@ -263,8 +265,9 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   pp.blk_base = 0;
   pp.any_flags = (int32_t*)(base + L.counter + 8);
   pp.PZ = (double*)(base + L.pz);
+  pp.PG = (int2*)(base + L.pg);
+  pp.PGZ = (float*)(base + L.pgz);
   pp.PXY = (double2*)(base + L.pxy);
-
   pp.PDZ2 = (double*)(base + L.pdz2);
   pp.PV = (ulonglong2*)(base + L.pv);
   pp.PKEY = (unsigned long long*)(base + L.pkey);
@@ -304,6 +307,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   fp.items = q.items;
   fp.n_items = q.n_items;
   fp.work_counter = (unsigned int*)(base + L.counter);
+  fp.PG = pp.PG; fp.PGZ = pp.PGZ;
   fp.PXY = pp.PXY; fp.PDZ2 = pp.PDZ2;
   fp.PV = pp.PV; fp.PKEY = pp.PKEY;
   fp.gkeys = (uint64_t*)(base + L.gkeys);

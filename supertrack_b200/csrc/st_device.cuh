@@ -5,13 +5,13 @@
 //   * prepared arena (written once per job, read once per oversample): for every job its kept
 //     deposits (those that can lie inside the voxel for some shift; in source order, grouped by
 //     cell inside each prepare block, or ordered by z layer) as a padded run of warp tiles of kWarpTile deposits.
-//     Lane l of a warp tile owns the kDepPerLane consecutive deposits 4l..4l+3 of the tile,
-//     stored "pair-blocked" (prep_slot in vcs_kernels.cu): the pair 4l, 4l+1 at tile slots
-//     2l, 2l+1 and the pair 4l+2, 4l+3 at 64+2l, 64+2l+1, so a warp reads one pair per lane with
-//     one 16-byte load per lane (512 contiguous bytes):
-//       PXY     : {x, y} as loaded, one 16-byte record per slot (padding slots hold NaN so the
-//                 box test rejects them); a lane's pair of slots is one 32-byte load
-//       PDZ2    : (k_z*d - a_z)^2, +inf when the deposit is outside the box in z
+//     Lane l of a warp tile owns the kDepPerLane consecutive deposits 4l..4l+3 of the tile:
+//       PG      : {X, Y} in lattice units, 8 bytes (set_integer_geometry; FP32 variant: float
+//                 {x, y}); a lane's four records are one 32-byte load
+//       PGZ     : the squared z distance from the layer's centres in the same units (float); a
+//                 lane's four are one 16-byte load
+//       PXY     : {x, y} as loaded, 16 bytes, and
+//       PDZ2    : (k_z*d - a_z)^2, read only for deposits that PG cannot decide
 //       PV      : v = edep / ((2/3) d) on the job's fixed-point grid, a 128-bit integer stored
 //                 as one 16-byte {low, high} record (one vector load per hit)
 //       PKEY    : k_z * N*N (the z part of the sphere key); bit 63 flags boundary deposits
@@ -19,7 +19,9 @@
 //     the CTA's shared-memory table (keys, 128-bit accumulators, used-slot list);
 //   * histograms: int64 counts and float64 y*f(y) sums per bin, one set per histogram.
 #pragma once
+#include <math.h>
 #include <stdint.h>
+#include <cmath>
 #include "st_core.cuh"
 
 namespace st {
@@ -76,7 +78,41 @@ struct JobDev {
   float f_inv_d;
   float f_r2;
   int32_t cell_nbr8;
+  // integer geometry of the FP64 form (set_integer_geometry)
+  double g_scale;     // 2^g_shift / d (0: every deposit is decided in FP64)
+  int32_t g_shift;
+  int32_t g_ns;       // N 2^g_shift
+  float g_lo, g_hi;   // squared distance at or below which a deposit hits, above which it misses
 };
+
+// Integer geometry: x and y of a deposit and the shift of an oversample in units of d / 2^s, rounded
+// to 32-bit integers. The position in the lattice is then V = X + C, with C the shift minus the
+// first sphere's centre plus half a cell: its high bits are the sphere index, its low s bits less
+// half a cell the offset from the centre, and the deposit is in the voxel when 0 < V < N 2^s.
+// X and C are each within 1/2 + 2^-20 unit of the exact value, so V is within 1.25 units. A
+// deposit is decided here only if it would be decided the same anywhere in that range: at least 2
+// units inside (or outside) the voxel's faces, and a squared distance (in units squared, with the
+// z part rounded to float) off the radius by more than `err` below: 2 (2 h 1.25 + 1.25^2) <
+// 5 h + 4 from x and y with h = 2^s / 2 the radius, and less than 2^-20 h^2 from four float
+// roundings of values near h^2. All others are decided by the FP64 arithmetic, so that hits and
+// sphere keys are the reference's bit for bit. N 2^s <= 2^30 keeps every V of a kept deposit
+// (|x| < 2HL') inside 32 bits; s <= 22 keeps the offsets exact in float. On a 5,000 nm voxel of
+// 2 nm spheres (s = 18) about 3e-5 of the deposits are near enough to a radius to need FP64.
+inline void set_integer_geometry(JobDev* D) {
+  int s = 22;
+  while (s > 0 && ((int64_t)D->N << s) > ((int64_t)1 << 30)) --s;
+  const double h = ldexp(0.5, s), err = 5.0 * h + 4.0 + h * h * 0x1p-20;
+  D->g_shift = s;
+  D->g_ns = (int32_t)((int64_t)D->N << s);
+  D->g_scale = ldexp(1.0 / D->d, s);
+  D->g_lo = nextafterf((float)(h * h - err), -INFINITY);
+  D->g_hi = nextafterf((float)(h * h + err), INFINITY);
+  if (!std::isfinite(D->g_scale) || !(D->g_scale >= 0x1p-1000)) {  // d outside the sane range
+    D->g_scale = 0.0;
+    D->g_lo = -1.0f;
+    D->g_hi = INFINITY;
+  }
+}
 
 // Deposits of a windowed job are processed in windows of consecutive kept deposits: kWindow (two
 // warp tiles per warp of the fused kernel's CTA), or twice that for jobs with coarse windows. A
@@ -151,8 +187,10 @@ struct FusedParams {
   const int* n_items;         // written by the planner
   int32_t flush_threshold;    // smem table occupancy that triggers a flush to the spill table
   unsigned int* work_counter; // next item to claim
-  const double2* PXY;         // {x, y} per slot (FP32 variant: float2 {x, y} at the slot's index)
-  const double* PDZ2;
+  const int2* PG;             // {X, Y} in lattice units (FP32 variant: float2 {x, y})
+  const float* PGZ;           // squared z distance, in lattice units (FP32 variant: nm)
+  const double2* PXY;         // {x, y} and
+  const double* PDZ2;         // (k_z d - a_z)^2 in FP64, for deposits that PG cannot decide
   const ulonglong2* PV;            // contribution on the job's grid: {low, high} 64-bit words
   const unsigned long long* PKEY;  // k_z * N*N, bit 63 = boundary deposit
   // spill tables: gridDim.x tables of gcap slots each
@@ -207,8 +245,10 @@ struct PrepareParams {
   int32_t win_tiles;          // warp tiles of a layer window (twice that on dense tracks)
   int32_t* any_flags;         // set when a job of the launch runs with window boundary flags
   double* PZ;                 // z after the z-origin shift (flagged jobs only)
-  double2* PXY;               // {x, y} per slot; FP32 variant: float2 {x, y} at the slot's index
-  double* PDZ2;               // FP32 variant: float dz^2 at the slot's float index
+  int2* PG;                   // records as in FusedParams; PXY and PDZ2 are not written in the
+  float* PGZ;                 // FP32 variant
+  double2* PXY;
+  double* PDZ2;
   ulonglong2* PV;
   unsigned long long* PKEY;
   int32_t fp32;               // 1: records for the FP32 geometry variant

@@ -41,7 +41,6 @@ __device__ __forceinline__ uint32_t table_hash(uint64_t key, uint32_t mask) {
 // ---------------------------------------------------------------------------------------------
 constexpr double kMagic = 0x1.8p52;             // adding it rounds |q| < 2^51 to an integer
 constexpr double kRiskBand = 0.5 - 0x1p-20;     // |q - rint(q)| at or above it: decide exactly
-constexpr int kGeoBlock = 2;                     // deposits per straight-line geometry block
 
 // The same, for one value: k = llrint(a / d) for |a / d| < 2^21.
 __device__ __forceinline__ double lattice_index(double a, double d, double inv_d) {
@@ -77,16 +76,8 @@ __device__ __forceinline__ int prep_job(const PrepareParams& p, int64_t b) {
   return p.blk_job ? __ldg(&p.blk_job[b]) - p.job_base : find_job(p.blk_prefix, p.n_jobs, b);
 }
 
-// Slot of kept deposit k of a job in the prepared arena: warp tiles of kWarpTile deposits in
-// which lane l owns deposits 4l..4l+3, stored "pair-blocked": the pair (4l, 4l+1) at tile slots
-// 2l, 2l+1 and the pair (4l+2, 4l+3) at 64 + 2l, 64 + 2l + 1. A warp reads a geometry block
-// (one pair per lane) with one 16-byte load per lane, 512 contiguous bytes per warp.
-__device__ __forceinline__ int64_t prep_slot(const JobDev& J, int64_t k) {
-  const int64_t w = k / kWarpTile;
-  const int rem = (int)(k - w * kWarpTile);
-  const int l = rem / kDepPerLane, pp = rem % kDepPerLane;
-  return J.prep_off + w * kWarpTile + (pp >> 1) * 64 + 2 * l + (pp & 1);
-}
+// Slot of kept deposit k of a job in the prepared arena.
+__device__ __forceinline__ int64_t prep_slot(const JobDev& J, int64_t k) { return J.prep_off + k; }
 
 // A windowed job whose kept deposits share cells (fewer than half as many occupied flag cells
 // of side d as deposits, or a quarter as many of side 2d: several hits per sphere) runs with
@@ -613,9 +604,13 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
       const double dz = st_dsub(st_dmul(kd, J.d), az);
       const int64_t dst = prep_slot(J, k);
       if (p.fp32) {
-        reinterpret_cast<float2*>(p.PXY)[dst] = make_float2(__double2float_rn(x[r]), __double2float_rn(y[r]));
-        reinterpret_cast<float*>(p.PDZ2)[dst] = __double2float_rn(st_dmul(dz, dz));
+        reinterpret_cast<float2*>(p.PG)[dst] = make_float2(__double2float_rn(x[r]), __double2float_rn(y[r]));
+        p.PGZ[dst] = __double2float_rn(st_dmul(dz, dz));
       } else {
+        const double gz = st_dmul(dz, J.g_scale);
+        p.PG[dst] = make_int2(__double2int_rn(st_dmul(x[r], J.g_scale)),
+                              __double2int_rn(st_dmul(y[r], J.g_scale)));
+        p.PGZ[dst] = __double2float_rn(st_dmul(gz, gz));
         p.PXY[dst] = make_double2(x[r], y[r]);
         p.PDZ2[dst] = st_dmul(dz, dz);
       }
@@ -708,13 +703,14 @@ __global__ void __launch_bounds__(kWarpTile) k_prep_pad(PrepareParams p) {
   if (k >= (kept / kWarpTile + 1) * kWarpTile) return;
   const int64_t dst = prep_slot(J, k);
   if (p.fp32) {
-    reinterpret_cast<float2*>(p.PXY)[dst] = make_float2(__int_as_float(0x7FC00000), __int_as_float(0x7FC00000));
-    reinterpret_cast<float*>(p.PDZ2)[dst] = __int_as_float(0x7F800000);
+    reinterpret_cast<float2*>(p.PG)[dst] = make_float2(__int_as_float(0x7FC00000), __int_as_float(0x7FC00000));
   } else {
+    p.PG[dst] = make_int2(INT_MIN, INT_MIN);  // outside the voxel for every shift
+    // (read when the job decides every deposit in FP64)
     p.PXY[dst] = make_double2(__longlong_as_double(0x7FF8000000000000ll),
                               __longlong_as_double(0x7FF8000000000000ll));
-    p.PDZ2[dst] = __longlong_as_double(0x7FF0000000000000ll);
   }
+  p.PGZ[dst] = __int_as_float(0x7F800000);
   p.PV[dst] = make_ulonglong2(0, 0);
   p.PKEY[dst] = 0;
 }
@@ -740,7 +736,7 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_flag(PrepareParams p) 
     const int64_t dst = prep_slot(J, k);
     double x, y;
     if (p.fp32) {  // float-rounded x, y: the FP32 jobs' cell size covers the rounding
-      const float2 xy = reinterpret_cast<const float2*>(p.PXY)[dst];
+      const float2 xy = reinterpret_cast<const float2*>(p.PG)[dst];
       x = xy.x;
       y = xy.y;
     } else {
@@ -832,11 +828,11 @@ __device__ __forceinline__ bool gtable_add(uint64_t* gk, unsigned long long* glo
   return false;
 }
 
-// {x, y} of two consecutive slots (32 bytes, 32-byte aligned: a lane's pair in a pair-blocked
-// tile) with one 256-bit read-only load.
-__device__ __forceinline__ void ldg_xy_pair(const double2* p, double* v) {
-  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-      : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
+// Four consecutive 8-byte records (32 bytes, 32-byte aligned: a lane's deposits of a tile) with one
+// 256-bit read-only load.
+__device__ __forceinline__ void ldg_records(const int2* p, unsigned long long* v) {
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
+      : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
       : "l"(p));
 }
 
@@ -893,6 +889,8 @@ struct CtaState {
   int logn;         // records in the spill log of this oversample
   int table;        // spill table that the CTA holds for its private items (-1: none)
   long long hist_work;  // deposit*oversamples in the shared-memory histogram
+  double sx, sy;      // shift of the current oversample, and in lattice units plus half a cell
+  int cx, cy;
 };
 
 // Spill table of the current item: the CTA's table restricted to a power-of-two prefix sized
@@ -1295,10 +1293,9 @@ __device__ __forceinline__ void log_reduce(const SmemTable<CAP>& T, CtaState& cs
 
 struct FusedJob {
   JobDev J;
+  int windowed;     // kWinNone, kWinFlags or kWinLayers
   const unsigned long long* wins;  // layered jobs: the window list, else null
-  int E0;
   int win_tiles;    // warp tiles per warp in a window: kWinTiles, or kCoarseTiles
-  int64_t n_wt;     // warp tiles of kept deposits
 };
 
 // Warp tiles of a shared unit's chunk: chunk_windows windows of kWinTiles tiles per warp,
@@ -1327,30 +1324,41 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
   constexpr int kWarps = THREADS / 32;
   const JobDev& J = F.J;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  float ux, uy;
-  shift_uniforms(J.seed, J.track_id, (uint32_t)os, J.shift_track, &ux, &uy);
-  const double sx = shift_from_uniform(ux, J.L, J.HL);
-  const double sy = shift_from_uniform(uy, J.L, J.HL);
-  const float sxf = __double2float_rn(sx), syf = __double2float_rn(sy);
+  const bool windowed = F.windowed != kWinNone;
+  const unsigned long long* const wins = F.wins;
+  const int64_t base = J.prep_off + 4 * lane;
+  const uint32_t N = J.N;
+  // F32: x' = x + sx, box |x'| < HL', a = x' - gSO, k = rint(a * (1/d)), dx = k*d - a,
+  // hit iff (dx^2 + dy^2) + dz^2 <= r^2, every step rounded to float
+  const float sxf = __double2float_rn(cs.sx), syf = __double2float_rn(cs.sy);
+  const float fHL = J.f_HL, fgSO = J.f_gSO, fd = J.f_d, finv = J.f_inv_d, fr2 = J.f_r2;
+  // FP64 form: integer geometry (set_integer_geometry). An offset below 2^22 becomes a float by
+  // its bits under the exponent of 2^23, less 2^23 and half a cell.
+  const int S = F32 ? 0 : J.g_shift;
+  const int cx = cs.cx, cy = cs.cy;
+  const unsigned in_max = (unsigned)J.g_ns - 4u, near_max = (unsigned)J.g_ns + 2u;
+  const unsigned low = (1u << S) - 1u;
+  const float centre = 8388608.0f + (float)(1 << S) * 0.5f;
+  const float lo2 = J.g_lo, hi2 = J.g_hi;
 
   // Jobs without window flags on the 8192-slot table run their windows without a barrier (a CTA
   // barrier per window cost more than the occasional new sphere sent to the spill table by a
   // full table); on the 4096-slot table, a job whose whole lattice (N^3 spheres) exceeds the flush
   // threshold checks the table at every window end and flushes it to the spill table
   const bool log_mode = cs.log_mode != 0;
-  const bool window_checks = CAP < 2 * kCtaTile && !J.flagged &&
+  const bool window_checks = CAP < 2 * kCtaTile && !windowed &&
                              (uint64_t)J.N * J.N2 > (uint64_t)P.flush_threshold;
   int wi = 0;  // emptied windows within this call
   bool logged = false;  // part of the current layer bin is in the spill log
   for (int64_t at = begin; at < end;) {
-    const int slot = J.flagged ? wi % 3 : 0;
+    const int slot = windowed ? wi % 3 : 0;
     // the window's warp tiles [w0, w1): win_tiles per warp from tile `at`, or window `at` of the
     // list, which may begin and end inside a tile (clip0: its first deposit in tile w0, clip1:
     // one past its last in tile w1 - 1)
     int w0, w1, clip0 = 0, clip1 = kWarpTile;
     bool more = false;  // the next window continues this one's last bin
-    if (F.wins) {
-      const unsigned long long a = __ldg(&F.wins[at]), b = __ldg(&F.wins[at + 1]);
+    if (wins) {
+      const unsigned long long a = __ldg(&wins[at]), b = __ldg(&wins[at + 1]);
       const long long k0 = (long long)(a & ~kWinContinues), k1 = (long long)(b & ~kWinContinues);
       more = (b & kWinContinues) != 0;
       w0 = (int)(k0 / kWarpTile);
@@ -1366,92 +1374,70 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
 #pragma unroll 1
     for (int w = w0 + warp; w < w1; w += kWarps) {
       {
-        // pair-blocked tile (prep_slot): this lane's deposits p = 0, 1 are the slots tb, tb + 1
-        // and p = 2, 3 the slots tb + 64, tb + 65
-        const int64_t tb = J.prep_off + (int64_t)w * kWarpTile + 2 * lane;
-        uint32_t kxv[kDepPerLane], kyv[kDepPerLane];
+        const int64_t tb = base + (int64_t)w * kWarpTile;  // this lane's deposits: tb .. tb + 3
+        int kxv[kDepPerLane], kyv[kDepPerLane];            // lattice indices, shifted by S
         unsigned hitmask = 0, boxmask = 0;
+        unsigned long long g[kDepPerLane];
+        ldg_records(P.PG + tb, g);
+        const float4 gz = __ldg(reinterpret_cast<const float4*>(P.PGZ + tb));
         if constexpr (F32) {
-          // x' = x + sx, box |x'| < HL', a = x' - gSO, k = rint(a * (1/d)), dx = k*d - a,
-          // hit iff (dx^2 + dy^2) + dz^2 <= r^2, every step rounded to float
-          const float2* pxy = reinterpret_cast<const float2*>(P.PXY) + tb;
-          const float* pdz = reinterpret_cast<const float*>(P.PDZ2) + tb;
-          const float4 xy01 = __ldg(reinterpret_cast<const float4*>(pxy));
-          const float4 xy23 = __ldg(reinterpret_cast<const float4*>(pxy + 64));
-          const float2 dz01 = __ldg(reinterpret_cast<const float2*>(pdz));
-          const float2 dz23 = __ldg(reinterpret_cast<const float2*>(pdz + 64));
-  #pragma unroll
+#pragma unroll
           for (int p = 0; p < kDepPerLane; ++p) {
-            const float2 xy = p == 0 ? make_float2(xy01.x, xy01.y) : p == 1 ? make_float2(xy01.z, xy01.w)
-                            : p == 2 ? make_float2(xy23.x, xy23.y) : make_float2(xy23.z, xy23.w);
-            const float dzp = p == 0 ? dz01.x : p == 1 ? dz01.y : p == 2 ? dz23.x : dz23.y;
-            const float x1 = __fadd_rn(xy.x, sxf);
-            const float y1 = __fadd_rn(xy.y, syf);
-            const bool inb = fabsf(x1) < J.f_HL && fabsf(y1) < J.f_HL;
+            const float z2 = p == 0 ? gz.x : p == 1 ? gz.y : p == 2 ? gz.z : gz.w;
+            const float x1 = __fadd_rn(__uint_as_float((unsigned)g[p]), sxf);
+            const float y1 = __fadd_rn(__uint_as_float((unsigned)(g[p] >> 32)), syf);
+            const bool inb = fabsf(x1) < fHL && fabsf(y1) < fHL;
             boxmask |= (unsigned)inb << p;
-            const float ax = __fsub_rn(x1, J.f_gSO);
-            const float ay = __fsub_rn(y1, J.f_gSO);
-            const int ix = __float2int_rn(__fmul_rn(ax, J.f_inv_d));
-            const int iy = __float2int_rn(__fmul_rn(ay, J.f_inv_d));
-            const float ddx = __fsub_rn(__fmul_rn((float)ix, J.f_d), ax);
-            const float ddy = __fsub_rn(__fmul_rn((float)iy, J.f_d), ay);
-            const float dist = __fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(ddy, ddy)), dzp);
-            hitmask |= (unsigned)(inb && dist <= J.f_r2) << p;
-            kxv[p] = (uint32_t)ix;
-            kyv[p] = (uint32_t)iy;
+            const float ax = __fsub_rn(x1, fgSO);
+            const float ay = __fsub_rn(y1, fgSO);
+            kxv[p] = __float2int_rn(__fmul_rn(ax, finv));
+            kyv[p] = __float2int_rn(__fmul_rn(ay, finv));
+            const float ddx = __fsub_rn(__fmul_rn((float)kxv[p], fd), ax);
+            const float ddy = __fsub_rn(__fmul_rn((float)kyv[p], fd), ay);
+            const float dist = __fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(ddy, ddy)), z2);
+            hitmask |= (unsigned)(inb && dist <= fr2) << p;
           }
         } else {
-        // geometry in straight-line blocks of kGeoBlock deposits, so their FP64 chains interleave
-  #pragma unroll
-        for (int h4 = 0; h4 < kDepPerLane; h4 += kGeoBlock) {
-          static_assert(kGeoBlock == 2, "a geometry block is a lane's pair of slots");
-          double ax[kGeoBlock], ay[kGeoBlock], kdx[kGeoBlock], kdy[kGeoBlock];
-          unsigned risk = 0;
-          double xy[4];  // x0, y0, x1, y1 of the pair: one 32-byte load
-          ldg_xy_pair(P.PXY + tb + h4 * 32, xy);
-  #pragma unroll
-          for (int p = 0; p < kGeoBlock; ++p) {
-            const double x1 = st_dadd(xy[2 * p], sx);
-            const double y1 = st_dadd(xy[2 * p + 1], sy);
-            const bool inb = fabs(x1) < J.HL && fabs(y1) < J.HL;
-            boxmask |= (unsigned)inb << (h4 + p);
-            ax[p] = st_dsub(x1, J.gSO);
-            ay[p] = st_dsub(y1, J.gSO);
-            const double qx = st_dmul(ax[p], J.inv_d);
-            const double qy = st_dmul(ay[p], J.inv_d);
-            kdx[p] = st_dsub(st_dadd(qx, kMagic), kMagic);
-            kdy[p] = st_dsub(st_dadd(qy, kMagic), kMagic);
-            const bool near_half = fabs(st_dsub(qx, kdx[p])) >= kRiskBand ||
-                                   fabs(st_dsub(qy, kdy[p])) >= kRiskBand;
-            risk |= (unsigned)(near_half && inb) << p;
+          unsigned undecided = 0;
+#pragma unroll
+          for (int p = 0; p < kDepPerLane; ++p) {
+            const float z2 = p == 0 ? gz.x : p == 1 ? gz.y : p == 2 ? gz.z : gz.w;
+            const int vx = (int)(unsigned)g[p] + cx, vy = (int)(unsigned)(g[p] >> 32) + cy;
+            const bool in = (unsigned)(vx - 2) <= in_max && (unsigned)(vy - 2) <= in_max;
+            const bool near = (unsigned)(vx + 1) <= near_max && (unsigned)(vy + 1) <= near_max;
+            const float fx = __fsub_rn(__uint_as_float(((unsigned)vx & low) | 0x4B000000u), centre);
+            const float fy = __fsub_rn(__uint_as_float(((unsigned)vy & low) | 0x4B000000u), centre);
+            const float d2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, z2));
+            const bool hit = in && d2 <= lo2;
+            boxmask |= (unsigned)in << p;
+            hitmask |= (unsigned)hit << p;
+            undecided |= (unsigned)(in ? (!hit && d2 <= hi2) : near) << p;
+            kxv[p] = vx;
+            kyv[p] = vy;
           }
-          if (risk) {
-            // q = RN(a * RN(1/d)) is within |q| 2^-51.2 of RN(a/d), far below 2^-20 for in-box
-            // quotients (|q| < 2^21); only a quotient this close to a half-integer can round
-            // differently, and then the IEEE division decides (rare: lattice-aligned inputs)
-  #pragma unroll
-            for (int p = 0; p < kGeoBlock; ++p) {
-              if (risk & (1u << p)) {
-                kdx[p] = rint(__ddiv_rn(ax[p], J.d));
-                kdy[p] = rint(__ddiv_rn(ay[p], J.d));
+          if (undecided) {
+            // the reference's arithmetic in FP64, each operation rounded on its own
+#pragma unroll
+            for (int p = 0; p < kDepPerLane; ++p) {
+              if (undecided & (1u << p)) {
+                const double2 xy = __ldg(&P.PXY[tb + p]);
+                const double x1 = st_dadd(xy.x, cs.sx), y1 = st_dadd(xy.y, cs.sy);
+                const bool inb = fabs(x1) < J.HL && fabs(y1) < J.HL;
+                boxmask = (boxmask & ~(1u << p)) | ((unsigned)inb << p);
+                if (inb) {
+                  const double ax = st_dsub(x1, J.gSO), ay = st_dsub(y1, J.gSO);
+                  const double kx = lattice_index(ax, J.d, J.inv_d), ky = lattice_index(ay, J.d, J.inv_d);
+                  const double dx = st_dsub(st_dmul(kx, J.d), ax), dy = st_dsub(st_dmul(ky, J.d), ay);
+                  const double dist = st_dadd(st_dadd(st_dmul(dx, dx), st_dmul(dy, dy)), __ldg(&P.PDZ2[tb + p]));
+                  hitmask |= (unsigned)(dist <= J.r2) << p;
+                  kxv[p] = __double2int_rn(kx) << S;
+                  kyv[p] = __double2int_rn(ky) << S;
+                }
               }
             }
           }
-          const double2 zb = __ldg(reinterpret_cast<const double2*>(P.PDZ2 + tb + h4 * 32));
-  #pragma unroll
-          for (int p = 0; p < kGeoBlock; ++p) {
-            const double ddx = st_dsub(st_dmul(kdx[p], J.d), ax[p]);
-            const double ddy = st_dsub(st_dmul(kdy[p], J.d), ay[p]);
-            const double dz2 = p == 0 ? zb.x : zb.y;
-            const double dist = st_dadd(st_dadd(st_dmul(ddx, ddx), st_dmul(ddy, ddy)), dz2);
-            const bool hit = ((boxmask >> (h4 + p)) & 1u) && dist <= J.r2;
-            hitmask |= (unsigned)hit << (h4 + p);
-            kxv[h4 + p] = (uint32_t)__double2loint(st_dadd(kdx[p], kMagic));
-            kyv[h4 + p] = (uint32_t)__double2loint(st_dadd(kdy[p], kMagic));
-          }
         }
-        }
-        if (F.wins) {  // lane's deposits 4 * lane + 0..3 of the tile that the window holds
+        if (wins) {  // lane's deposits 4 * lane + 0..3 of the tile that the window holds
           unsigned in = 0xFu;
           if (w == w0) in &= 0xFu << min(max(clip0 - 4 * lane, 0), 4);
           if (w == w1 - 1) in &= (1u << min(max(clip1 - 4 * lane, 0), 4)) - 1u;
@@ -1466,15 +1452,16 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
   #pragma unroll
         for (int p = 0; p < kDepPerLane; ++p) {
           if (hitmask & (1u << p)) {
-            const int64_t idx = tb + (p >> 1) * 64 + (p & 1);
+            const int64_t idx = tb + p;
             const ulonglong2 v = __ldg(&P.PV[idx]);
             const uint64_t lo = v.x;
             const uint64_t hi = v.y;
             const uint64_t kzw = __ldg(&P.PKEY[idx]);
             // (the FP32 form converts a lattice index like the reference's llrint: sign-extended)
             const uint64_t key =
-                (F32 ? (uint64_t)(int64_t)(int32_t)kxv[p] + (uint64_t)(int64_t)(int32_t)kyv[p] * J.N
-                     : (uint64_t)kxv[p] + (uint64_t)kyv[p] * J.N) + (kzw & ~kBoundaryBit);
+                (F32 ? (uint64_t)(int64_t)kxv[p] + (uint64_t)(int64_t)kyv[p] * N
+                     : (uint64_t)(uint32_t)(kxv[p] >> S) + (uint64_t)(uint32_t)(kyv[p] >> S) * N) +
+                (kzw & ~kBoundaryBit);
             const bool bflag = (kzw & kBoundaryBit) != 0;
             if (key == rkey) {
               add128(rlo, rhi, lo, hi);
@@ -1493,7 +1480,7 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
         if (rkey != kEmptyKey) sphere_add<CAP>(T, &cs, P, G, rkey, rlo, rhi, rflag, slot);
       }
     }
-    if (J.flagged) {
+    if (windowed) {
       // window done: spheres without boundary contributions are complete -> bin them now;
       // the others (or all, if the window overflowed) go to the spill table
       __syncthreads();
@@ -1584,6 +1571,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
   __shared__ int s_bcast[2];
   __shared__ BinContext sB;   // the item's binning context and spill table, uniform over the
   __shared__ Spill sG;        // CTA: kept in shared memory rather than in every thread's registers
+  __shared__ FusedJob sF;     // (likewise the job)
 
   const int HB = P.smem_hist_bins;
   const SmemTable<CAP> T;
@@ -1621,13 +1609,19 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     const WorkItem W = P.items[it];
     const JobAux A = P.aux[W.job];
     if (A.flags & kAuxNonfinite) continue;  // rejected job: contributes nothing, host reports it
-    FusedJob F;
-    F.J = P.jobs[W.job];
-    F.J.flagged = A.windowed;  // window flags and lists were computed only for these jobs
-    F.wins = A.windowed == kWinLayers ? P.wins + F.J.win_off : nullptr;
-    F.win_tiles = coarse_windows(F.J, A) ? kCoarseTiles : kWinTiles;
-    F.E0 = choose_grid_exponent(A.e_min, A.e_max, F.J.n, A.flags & kAuxNonzero);
-    F.n_wt = (A.kept + kWarpTile - 1) / kWarpTile;
+    static_assert(sizeof(JobDev) % 8 == 0, "copied by 64-bit words");
+    if (tid < (int)(sizeof(JobDev) / 8))
+      reinterpret_cast<unsigned long long*>(&sF.J)[tid] =
+          reinterpret_cast<const unsigned long long*>(&P.jobs[W.job])[tid];
+    __syncthreads();
+    const FusedJob& F = sF;
+    const int E0 = choose_grid_exponent(A.e_min, A.e_max, F.J.n, A.flags & kAuxNonzero);
+    const int64_t n_wt = (A.kept + kWarpTile - 1) / kWarpTile;
+    if (tid == 0) {
+      sF.windowed = A.windowed;
+      sF.wins = A.windowed == kWinLayers ? P.wins + F.J.win_off : nullptr;
+      sF.win_tiles = coarse_windows(F.J, A) ? kCoarseTiles : kWinTiles;
+    }
     const HistDev H = P.hists[F.J.hist];
     const bool smem_hist = H.nbins <= HB;
 
@@ -1659,7 +1653,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
       sB.mode = H.mode;
       sB.ca = H.ca;
       sB.cb = H.cb;
-      sB.E0 = F.E0;
+      sB.E0 = E0;
       sB.job = W.job;
       sB.hcount = smem_hist ? hcount : nullptr;
       sB.hylo = smem_hist ? hylo : nullptr;
@@ -1676,7 +1670,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     // helper claims window chunks of its shared unit until none is left.
     const bool shared = W.unit >= 0;
     const int64_t wpc = chunk_tiles(P.chunk_windows);  // warp tiles per chunk
-    const int64_t n_chunks = (F.n_wt + wpc - 1) / wpc;
+    const int64_t n_chunks = (n_wt + wpc - 1) / wpc;
     // A private item's spill table stays with the CTA for its next private items; it goes back to
     // the pool before the CTA joins a shared unit, so that a CTA holds at most one.
     if (tid == 0) {
@@ -1698,7 +1692,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
         os = W.os_begin + seg;
         t = private_table;
         wb = 0;
-        we = F.n_wt;
+        we = n_wt;
         if (F.wins) {
           // whole bins: a window that continues a bin belongs to the item that began it
           wb = W.win_begin;
@@ -1719,17 +1713,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
         if (c < 0 || t < 0) break;
         os = W.os_begin;
         wb = (int64_t)c * wpc;
-        we = wb + wpc < F.n_wt ? wb + wpc : F.n_wt;
+        we = wb + wpc < n_wt ? wb + wpc : n_wt;
       }
       if (tid == 0) {
         sG = spill_of(P, t, A.kept);
         cs.log_mode = !shared;  // a single CTA sees every window of the oversample
+        const JobDev& J = F.J;
+        float ux, uy;
+        shift_uniforms(J.seed, J.track_id, (uint32_t)os, J.shift_track, &ux, &uy);
+        cs.sx = shift_from_uniform(ux, J.L, J.HL);
+        cs.sy = shift_from_uniform(uy, J.L, J.HL);
+        const int half = 1 << J.g_shift >> 1;
+        cs.cx = __double2int_rn(st_dmul(st_dsub(cs.sx, J.gSO), J.g_scale)) + half;
+        cs.cy = __double2int_rn(st_dmul(st_dsub(cs.sy, J.gSO), J.g_scale)) + half;
       }
       __syncthreads();
       const Spill& G = sG;
       superimpose<CAP, THREADS, F32>(P, F, T, cs, G, B, os, wb, we, hits, inbox, spheres, binned);
       if (cs.log_mode) {
-        if (!F.J.flagged && cs.logn > 0) {
+        if (!F.windowed && cs.logn > 0) {
           // the table's spheres may have parts in the log: they join it
           flush_to_log<CAP, THREADS>(T, cs.tc[0], &cs, P, G);
           __syncthreads();
@@ -1738,7 +1740,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
         }
         log_reduce<CAP, THREADS>(T, cs, P, G, B, spheres, binned, os);
       }
-      const int cnt = F.J.flagged ? 0 : cs.tc[0];  // flagged windows leave the table empty
+      const int cnt = F.windowed ? 0 : cs.tc[0];  // flagged windows leave the table empty
       bool bin_table;
       if (!shared) {
         bin_table = cs.spilled != 0;
