@@ -25,7 +25,8 @@ cudaError_t launch_unit_wait_probe(int* table, int* error_flags, int* out, long 
                                    cudaStream_t s);
 cudaError_t launch_smem_atomic_probe(unsigned long long* out, int blocks, int iters, cudaStream_t s);
 cudaError_t launch_plan(const PlanParams& q, cudaStream_t s);
-cudaError_t launch_reset_aux(JobAux* aux, int n, cudaStream_t s);
+cudaError_t launch_reset(const ResetParams& p, cudaStream_t s);
+int plan_launches(int n_jobs);
 }  // namespace st
 
 namespace {
@@ -615,6 +616,26 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   return ST_OK;
 }
 
+// What a run of nj jobs resets on the device (launch_reset).
+st::ResetParams reset_params(st_ctx* c, size_t nj, bool want_export) {
+  st::ResetParams r{};
+  r.aux = (JobAux*)c->d_aux.p;
+  r.n_jobs = (int32_t)nj;
+  r.counter = (unsigned int*)c->d_counter.p;
+  r.pool = (unsigned int*)c->pool.p;
+  r.n_pool = (c->cache_grid + 31) / 32;
+  r.plan = (unsigned int*)c->d_plan_misc.p;
+  r.u_next = (unsigned int*)c->u_next.p;
+  r.u_done = (unsigned int*)c->u_done.p;
+  r.u_table = (unsigned int*)c->u_table.p;
+  r.n_units = c->cache_units;
+  r.bins = (uint32_t*)c->z_bins.p;
+  r.n_bins = c->cache_bins;
+  r.err = (unsigned int*)c->d_err.p;
+  r.ex_count = want_export ? (unsigned int*)c->ex_count.p : nullptr;
+  return r;
+}
+
 // Enqueues the device side of a run on the context's stream: the resets, the prepare, plan and
 // fused kernels, and the copies of the job counters and error flags into pinned host memory,
 // with the run's events. Nothing waits; finish_range picks the results up. While the stream is
@@ -622,20 +643,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
 st_status enqueue_run(st_ctx* c, const st::FusedParams& fp, size_t nj, bool want_export,
                       bool capturing) {
   const unsigned evf = capturing ? cudaEventRecordExternal : cudaEventRecordDefault;
-  ST_CUDA(st::launch_reset_aux((JobAux*)c->d_aux.p, (int)nj, c->stream), "reset aux");
-  ST_CUDA(cudaMemsetAsync(c->d_counter.p, 0, 16, c->stream), "reset counter");
-  if (c->cache_grid > 0)
-    ST_CUDA(cudaMemsetAsync(c->pool.p, 0, (size_t)((c->cache_grid + 31) / 32) * 4, c->stream), "pool reset");
-  ST_CUDA(cudaMemsetAsync(c->d_plan_misc.p, 0, 16 + 3 * 4 * st::kPlanBuckets, c->stream), "plan reset");
-  if (c->cache_units > 0) {
-    ST_CUDA(cudaMemsetAsync(c->u_next.p, 0, (size_t)c->cache_units * 4, c->stream), "unit reset");
-    ST_CUDA(cudaMemsetAsync(c->u_done.p, 0, (size_t)c->cache_units * 4, c->stream), "unit reset");
-    ST_CUDA(cudaMemsetAsync(c->u_table.p, 0xFF, (size_t)c->cache_units * 4, c->stream), "unit reset");
-  }
-  if (c->cache_bins > 0)
-    ST_CUDA(cudaMemsetAsync(c->z_bins.p, 0, (size_t)c->cache_bins * 4, c->stream), "z bin reset");
-  ST_CUDA(cudaMemsetAsync(c->d_err.p, 0, 16, c->stream), "reset errors");
-  if (want_export) ST_CUDA(cudaMemsetAsync(c->ex_count.p, 0, 16, c->stream), "export counter");
+  ST_CUDA(st::launch_reset(reset_params(c, nj, want_export), c->stream), "reset");
 
   ST_CUDA(cudaEventRecordWithFlags(c->ev[0], c->stream, evf), "event");
   ST_CUDA(st::launch_prepare(c->cache_pp, c->cache_blocks, c->cache_any_flagged, c->stream), "prepare launch");
@@ -663,23 +671,17 @@ st_status enqueue_run(st_ctx* c, const st::FusedParams& fp, size_t nj, bool want
 st_status enqueue_groups(st_ctx* c, const st::FusedParams& fp, size_t first,
                          const std::vector<size_t>& groups) {
   const size_t nj = groups.back() - first;
-  ST_CUDA(st::launch_reset_aux((JobAux*)c->d_aux.p, (int)nj, c->stream), "reset aux");
-  if (c->cache_bins > 0)
-    ST_CUDA(cudaMemsetAsync(c->z_bins.p, 0, (size_t)c->cache_bins * 4, c->stream), "z bin reset");
-  ST_CUDA(cudaMemsetAsync(c->d_err.p, 0, 16, c->stream), "reset errors");
+  st::ResetParams reset = reset_params(c, nj, false);
+  ST_CUDA(st::launch_reset(reset, c->stream), "reset");
+  // a later group resets what the launches of a group share
+  reset.n_jobs = 0;
+  reset.n_bins = 0;
+  reset.err = nullptr;
   ST_CUDA(cudaEventRecord(c->ev[0], c->stream), "event");
   for (size_t g = 0; g + 1 < groups.size(); ++g) {
     const size_t j0 = groups[g] - first, j1 = groups[g + 1] - first;
     ST_CUDA(cudaStreamWaitEvent(c->stream, c->up_ev[g], 0), "upload wait");
-    ST_CUDA(cudaMemsetAsync(c->d_counter.p, 0, 16, c->stream), "reset counter");
-    if (c->cache_grid > 0)
-      ST_CUDA(cudaMemsetAsync(c->pool.p, 0, (size_t)((c->cache_grid + 31) / 32) * 4, c->stream), "pool reset");
-    ST_CUDA(cudaMemsetAsync(c->d_plan_misc.p, 0, 16 + 3 * 4 * st::kPlanBuckets, c->stream), "plan reset");
-    if (c->cache_units > 0) {
-      ST_CUDA(cudaMemsetAsync(c->u_next.p, 0, (size_t)c->cache_units * 4, c->stream), "unit reset");
-      ST_CUDA(cudaMemsetAsync(c->u_done.p, 0, (size_t)c->cache_units * 4, c->stream), "unit reset");
-      ST_CUDA(cudaMemsetAsync(c->u_table.p, 0xFF, (size_t)c->cache_units * 4, c->stream), "unit reset");
-    }
+    if (g > 0) ST_CUDA(st::launch_reset(reset, c->stream), "reset");
     st::PrepareParams pp = c->cache_pp;
     pp.jobs += j0;
     pp.aux += j0;
@@ -867,9 +869,9 @@ st_status launch_range(st_ctx* c, size_t first, size_t last, bool want_export, i
     if (s != ST_OK) return s;
   }
   const size_t n_groups = groups.size() - 1;
-  c->launches += (nj > 0 ? 1 : 0) +
-                 (int32_t)n_groups * ((c->cache_blocks > 0 ? (c->cache_any_flagged ? 6 : 4) : 0) +
-                                      (nj > 0 ? 4 : 0) + (c->cache_grid > 0 ? 1 : 0));
+  for (size_t g = 0; g < n_groups; ++g)
+    c->launches += 1 + (c->cache_blocks > 0 ? (c->cache_any_flagged ? 6 : 4) : 0) +
+                   st::plan_launches((int)(groups[g + 1] - groups[g])) + (c->cache_grid > 0 ? 1 : 0);
   c->pending = true;
   c->pend_first = first;
   c->pend_last = last;

@@ -8,7 +8,7 @@
 // of the library image.
 //
 // The scratch below is a file-scope __device__ array: every GPU that loads the library holds it
-// (kScratchBytes, about 6.2 MB) until the process exits. Host code cannot pass the symbol
+// (kScratchBytes, about 6.9 MB) until the process exits. Host code cannot pass the symbol
 // itself to a kernel (on the host it names a host-side stand-in), so the first call on each
 // device, with that device current, resolves its device address with cudaGetSymbolAddress and
 // sets the fused kernel's shared-memory attribute; that first call should therefore come before
@@ -36,6 +36,7 @@ cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_fl
 cudaError_t configure_fused();
 cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s);
 cudaError_t launch_plan(const PlanParams& q, cudaStream_t s);
+cudaError_t launch_reset(const ResetParams& p, cudaStream_t s);
 }  // namespace st
 
 namespace {
@@ -43,7 +44,8 @@ namespace {
 constexpr int64_t kNaMaxDeposits = 16384;       // deposits per track
 constexpr int32_t kNaMaxBins = 4096;            // histogram bins
 constexpr int64_t kNaMaxOversamples = 65536;    // oversamples per call
-constexpr int kNaGrid = 4;                      // resident CTAs (and spill tables)
+constexpr int kNaGrid = 4;                      // spill tables of the largest track's size; a
+                                                // smaller track has more CTAs, with smaller tables
 constexpr uint32_t kNaTableCap = 2 * kNaMaxDeposits;   // spill-table slots (power of two)
 constexpr uint32_t kNaCellCap = 2 * kNaMaxDeposits;    // cell-hash slots (power of two)
 constexpr int64_t kNaBlocks = kNaMaxDeposits / st::kPrepSlotsPerBlock;
@@ -85,7 +87,7 @@ constexpr Layout make_layout() {
   L.glo = o;        o += al((size_t)kNaGrid * kNaTableCap * 8);
   L.ghi = o;        o += al((size_t)kNaGrid * kNaTableCap * 8);
   L.gused = o;      o += al((size_t)kNaGrid * kNaTableCap * 4);
-  L.gcount = o;     o += al((size_t)kNaGrid * 4);
+  L.gcount = o;     o += al(32 * 4);
   L.pool = o;       o += al(4);
   L.items = o;      o += al((size_t)kNaMaxOversamples * sizeof(st::WorkItem));
   L.plan = o;       o += al(sizeof(st::JobPlan));
@@ -208,11 +210,6 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   D.inv_cell = 1.0 / D.cell_size;
   st::set_integer_geometry(&D);
 
-  st::JobAux A;
-  std::memset(&A, 0, sizeof(A));
-  A.e_min = INT_MAX;
-  A.e_max = INT_MIN;
-
   st::HistDev H;
   std::memset(&H, 0, sizeof(H));
   H.edges = (const double*)(base + L.edges);
@@ -237,21 +234,37 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   } while (0)
 
   NA_CUDA(cudaMemcpyAsync(base + L.jobs, &D, sizeof(D), cudaMemcpyHostToDevice, st_));
-  NA_CUDA(cudaMemcpyAsync(base + L.aux, &A, sizeof(A), cudaMemcpyHostToDevice, st_));
   NA_CUDA(cudaMemcpyAsync(base + L.hists, &H, sizeof(H), cudaMemcpyHostToDevice, st_));
   NA_CUDA(cudaMemcpyAsync(base + L.blk_prefix, blk, sizeof(blk), cudaMemcpyHostToDevice, st_));
   NA_CUDA(cudaMemcpyAsync(base + L.edges, edges, (size_t)(nbins + 1) * 8, cudaMemcpyHostToDevice, st_));
-  // everything that must start empty: hash tables, counters, flags
-  NA_CUDA(cudaMemsetAsync(base + L.gkeys, 0xFF, (size_t)kNaGrid * kNaTableCap * 8, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.glo, 0, (size_t)kNaGrid * kNaTableCap * 8, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.ghi, 0, (size_t)kNaGrid * kNaTableCap * 8, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.gcount, 0, (size_t)kNaGrid * 4, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.pool, 0, 4, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.plan_misc, 0, 16 + 3 * 4 * st::kPlanBuckets, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.counter, 0, 16, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.err, 0, 16, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.units, 0, 8, st_));
-  NA_CUDA(cudaMemsetAsync(base + L.units + 8, 0xFF, 4, st_));
+  // Spill tables: as many as the scratch holds of the size that this track needs (its deposits
+  // twice, as in the regular path), one per CTA and at most the pool's 32. (Sixteen CTAs instead
+  // of four for a track of 4,000 deposits, its items sized for them, and one reset kernel in place
+  // of eleven memsets: 148 -> 100 us for 10 oversamples.)
+  uint32_t gcap = 1024;
+  while ((int64_t)gcap < 2 * n_pad && gcap < (uint32_t)kNaTableCap) gcap <<= 1;
+  const int grid = (int)std::min<int64_t>(32, (int64_t)kNaGrid * kNaTableCap / gcap);
+  // everything that must start empty: hash tables, counters, flags, the job's counters
+  st::ResetParams r;
+  std::memset(&r, 0, sizeof(r));
+  r.aux = (st::JobAux*)(base + L.aux);
+  r.n_jobs = 1;
+  r.counter = (unsigned int*)(base + L.counter);
+  r.pool = (unsigned int*)(base + L.pool);
+  r.n_pool = 1;
+  r.plan = (unsigned int*)(base + L.plan_misc);
+  r.u_next = (unsigned int*)(base + L.units);
+  r.u_done = (unsigned int*)(base + L.units + 4);
+  r.u_table = (unsigned int*)(base + L.units + 8);
+  r.n_units = 1;
+  r.err = (unsigned int*)(base + L.err);
+  r.gkeys = (uint64_t*)(base + L.gkeys);
+  r.glo = (unsigned long long*)(base + L.glo);
+  r.ghi = (unsigned long long*)(base + L.ghi);
+  r.gcount = (unsigned int*)(base + L.gcount);
+  r.n_slots = (int64_t)grid * gcap;
+  r.n_tables = grid;
+  NA_CUDA(st::launch_reset(r, st_));
 
   st::PrepareParams pp;
   std::memset(&pp, 0, sizeof(pp));
@@ -284,10 +297,10 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   q.n_jobs = 1;
   q.chunk_windows = kNaChunkWindows;
   q.max_helpers = 1;
-  q.grid = kNaGrid;
+  q.grid = grid;
   q.item_cost = kNaItemCost;
   // deliberate difference from the regular path: share_divisor 0 (left zero) rules out shared
-  // units, whose helpers would need a spill table each from a pool sized for kNaGrid CTAs;
+  // units, whose helpers would need a spill table each from a pool of one table per CTA;
   // min_chunks only matters for shared units
   q.total_units = (unsigned long long*)m;
   q.n_items = (int*)(m + 8);
@@ -315,7 +328,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   fp.ghi = (unsigned long long*)(base + L.ghi);
   fp.gused = (uint32_t*)(base + L.gused);
   fp.gcount = (unsigned int*)(base + L.gcount);
-  fp.gcap = kNaTableCap;
+  fp.gcap = gcap;
   fp.error_flags = (int*)(base + L.err);
   fp.unit_next = (unsigned int*)(base + L.units);
   fp.unit_done = (unsigned int*)(base + L.units + 4);
@@ -325,7 +338,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
 
   NA_CUDA(st::launch_prepare(pp, n_blocks, D.flagged != 0, st_));
   NA_CUDA(st::launch_plan(q, st_));
-  NA_CUDA(st::launch_fused(fp, nbins, kNaGrid, 0, st_));
+  NA_CUDA(st::launch_fused(fp, nbins, grid, 0, st_));
 
   // ---- status: job counters and device error flags (host stack destinations)
   st::JobAux out;

@@ -289,6 +289,32 @@ struct PlanParams {
   long long item_cap;
 };
 
+// A run's state on the device that starts from fixed values, set by one kernel (launch_reset).
+struct ResetParams {
+  JobAux* aux;                 // n_jobs job records: exponent range empty, everything else zero
+  int32_t n_jobs;
+  int32_t n_pool;
+  unsigned int* counter;       // 4 words of zeros: work counter, any_flags
+  unsigned int* pool;          // n_pool words of zeros
+  unsigned int* plan;          // the planner's scratch, kPlanScratch bytes of zeros
+  unsigned int* u_next;        // n_units words each: zeros, zeros, all ones
+  unsigned int* u_done;
+  unsigned int* u_table;
+  int64_t n_units;
+  uint32_t* bins;              // n_bins words of zeros
+  int64_t n_bins;
+  unsigned int* err;           // 4 words of zeros (null: kept)
+  unsigned int* ex_count;      // 4 words of zeros (null: none)
+  // empty spill tables (null: kept): n_slots keys of ones and sums of zeros, n_tables counters
+  uint64_t* gkeys;
+  unsigned long long* glo;
+  unsigned long long* ghi;
+  unsigned int* gcount;
+  int64_t n_slots;
+  int32_t n_tables;
+};
+constexpr int kPlanScratch = 16 + 3 * 4 * kPlanBuckets;  // bytes
+
 constexpr int kPrepThreads = 256;
 constexpr int kPrepSlotsPerBlock = 1024;                // source deposits per prepare block
 constexpr int kFusedWarps = 32;                       // warps of the fused kernel's CTA

@@ -4,7 +4,7 @@
 //               can be in the voxel for some shift, the z part of the lattice test (k_z and
 //               (k_z*d - a_z)^2, which do not depend on the oversample), the lineal energy
 //               contribution v = edep/((2/3)d), the job's fixed-point exponent range, and the
-//               ordered compaction of the kept deposits into the pair-blocked prepared arena.
+//               ordered compaction of the kept deposits into the prepared arena.
 //               Follows VoxelConstrainedSphereMethod.cu:138-154 (z shift), :198 (|z| test),
 //               :249-258 (z axis of the membership test), :302/:322 (lineal denominator).
 //   k_fused   : persistent work-stealing kernel over (job, oversample block) items. Per
@@ -56,7 +56,7 @@ __device__ __forceinline__ double lattice_index(double a, double d, double inv_d
 //                  strictly inside; |x|, |y| below xy_keep), plus the job's exponent range of
 //                  the contributions v = edep/((2/3)d) over all its deposits;
 //   k_prep_scan  : per job, exclusive scan of its block counts -> block offsets, kept total;
-//   k_prep_write : ordered compaction of the kept deposits into the pair-blocked arena with
+//   k_prep_write : ordered compaction of the kept deposits into the prepared arena with
 //                  the oversample-independent z part of the lattice test;
 //   k_prep_pad   : padding of each job's last warp tile (NaN x so the box test rejects it).
 // A dropped deposit can be inside the box for no shift, so dropping it changes no result.
@@ -1857,18 +1857,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
 // Planner (after the prepare stage, before k_fused): work items from the kept deposit counts.
 // A job whose kept deposits per oversample exceed both min_chunks chunks (4) and 1/share_divisor
 // (1/8) of one CTA's share of the batch runs as shared units (one per oversample, `helpers` helper items each);
-// every other job runs as private items of about item_cost deposit*oversamples. Items are
+// every other job runs as private items (plan_item_cost), a layered job's also as parts of an
+// oversample. Items are
 // bucketed by cost, largest first (longest-processing-time order at bucket granularity).
 // ---------------------------------------------------------------------------------------------
-__global__ void k_plan_total(PlanParams q) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned long long v = 0;
-  if (j < q.n_jobs) v = (unsigned long long)q.aux[j].kept * (unsigned long long)q.jobs[j].n_os;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0 && v) atomicAdd(q.total_units, v);
-}
-
 __device__ __forceinline__ int cost_bucket(long long cost) {
   int l = 0;
   while (cost > 1 && l < 62) { cost >>= 1; ++l; }
@@ -1881,16 +1873,14 @@ __device__ __forceinline__ int cost_bucket(long long cost) {
 // 0.40 ms, against 0.062 ms split; a track of 10 oversamples, one at a time, 84 -> 25 us. A half
 // instead of an eighth of the share made groups of uneven tracks wait for their largest items
 // (6.2 against 5.6 ms for 256 host tracks in groups).
-__device__ __forceinline__ long long plan_item_cost(const PlanParams& q) {
-  const long long share = (long long)(*q.total_units / ((unsigned long long)q.grid * 8));
+__device__ __forceinline__ long long plan_item_cost(const PlanParams& q, unsigned long long total_units) {
+  const long long share = (long long)(total_units / ((unsigned long long)q.grid * 8));
   const long long lo = 2048;
   const long long ic = share < lo ? lo : share;
   return ic < q.item_cost ? ic : q.item_cost;
 }
 
-__global__ void k_plan_size(PlanParams q) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= q.n_jobs) return;
+__device__ __forceinline__ JobPlan plan_job(const PlanParams& q, int j, unsigned long long total_units) {
   const long long kept = q.aux[j].kept;
   const long long nos = q.jobs[j].n_os;
   JobPlan pl;
@@ -1902,12 +1892,12 @@ __global__ void k_plan_size(PlanParams q) {
   if (kept > 0 && nos > 0 && !(q.aux[j].flags & kAuxNonfinite)) {
     const long long chunk = chunk_tiles(q.chunk_windows) * kWarpTile;
     const long long share =
-        q.share_divisor > 0 ? (long long)(*q.total_units / ((unsigned long long)q.share_divisor * q.grid)) : 0;
+        q.share_divisor > 0 ? (long long)(total_units / ((unsigned long long)q.share_divisor * q.grid)) : 0;
     if (q.aux[j].windowed == kWinLayers) {
       // any range of windows is complete on its own: about item_cost of work per item, as whole
       // oversamples or as parts of one
       const long long n_win = q.aux[j].n_win;
-      const long long ic = plan_item_cost(q);
+      const long long ic = plan_item_cost(q, total_units);
       if (kept > ic && n_win > 1) {
         long long parts = (kept + ic - 1) / ic;
         parts = parts < q.max_helpers ? parts : q.max_helpers;
@@ -1934,39 +1924,22 @@ __global__ void k_plan_size(PlanParams q) {
       pl.bucket = cost_bucket(kept);
     } else {
       const long long pad = ((kept + kWarpTile - 1) / kWarpTile) * kWarpTile;
-      long long b = plan_item_cost(q) / pad;
+      long long b = plan_item_cost(q, total_units) / pad;
       b = b < 1 ? 1 : (b > nos ? nos : b);
       pl.blk_os = (int)b;
       pl.items = (int)((nos + b - 1) / b);
       pl.bucket = cost_bucket(pad * b);
     }
-    atomicAdd(&q.bucket_count[pl.bucket], (unsigned)pl.items);
   }
-  q.plan[j] = pl;
+  return pl;
 }
 
-__global__ void k_plan_scan(PlanParams q) {
-  if (threadIdx.x != 0) return;
-  unsigned run = 0;
-  for (int b = 0; b < kPlanBuckets; ++b) {
-    q.bucket_start[b] = run;
-    q.bucket_cursor[b] = 0;
-    run += q.bucket_count[b];
-  }
-  *q.n_items = (long long)run <= q.item_cap ? (int)run : (int)q.item_cap;
-}
-
-__global__ void __launch_bounds__(128) k_plan_write(PlanParams q) {
-  const int j = blockIdx.x;
-  const JobPlan pl = q.plan[j];
-  if (pl.items == 0) return;
-  __shared__ unsigned s_pos;
-  if (threadIdx.x == 0)
-    s_pos = q.bucket_start[pl.bucket] + atomicAdd(&q.bucket_cursor[pl.bucket], (unsigned)pl.items);
-  __syncthreads();
+// Items of job j, by the threads i = first, first + step, ... of the caller, from position `at`.
+__device__ __forceinline__ void plan_items(const PlanParams& q, int j, const JobPlan& pl, long long at,
+                                           int first, int step) {
   const int nos = q.jobs[j].n_os;
-  for (int k = threadIdx.x; k < pl.items; k += blockDim.x) {
-    const long long pos = (long long)s_pos + k;
+  for (int k = first; k < pl.items; k += step) {
+    const long long pos = at + k;
     if (pos >= q.item_cap) break;
     WorkItem w;
     w.job = j;
@@ -1995,41 +1968,123 @@ __global__ void __launch_bounds__(128) k_plan_write(PlanParams q) {
   }
 }
 
-// Job counters of a run to their initial values (exponent range empty, everything else zero).
-// A kernel rather than a copy from the host: a host-to-device copy on the run's stream would queue
-// on a copy engine behind any track upload in flight and hold the run's kernels back.
-__global__ void k_reset_aux(JobAux* aux, int n) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  JobAux a;
-  a.e_min = INT_MAX;
-  a.e_max = INT_MIN;
-  a.flags = 0;
-  a.windowed = 0;
-  a.kept = 0;
-  a.hits = 0;
-  a.spheres = 0;
-  a.binned = 0;
-  a.inbox = 0;
-  a.cells = 0;
-  a.n_win = 0;
-  a.reserved = 0;
-  aux[j] = a;
+// One CTA: the batch's work, every job's plan, the buckets' places in the item list and, for up to
+// kPlanSmall jobs, the items themselves (k_plan_write writes those of larger batches). One launch
+// instead of the four that these steps were: a dependent launch costs a small batch 3 to 5 us.
+// With k_reset for the memsets: one proton track of 19,997 deposits 214 -> 181 us per pass, 16 short
+// tracks one at a time 2.10 -> 1.63 ms, 64 in a batch 286 -> 269 us.
+constexpr int kPlanSmall = 64;
+__global__ void __launch_bounds__(1024) k_plan(PlanParams q) {
+  __shared__ unsigned long long s_total;
+  __shared__ unsigned s_count[kPlanBuckets], s_start[kPlanBuckets];
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) s_total = 0;
+  if (tid < kPlanBuckets) s_count[tid] = 0;
+  __syncthreads();
+  unsigned long long v = 0;
+  for (int j = tid; j < q.n_jobs; j += 1024)
+    v += (unsigned long long)q.aux[j].kept * (unsigned long long)q.jobs[j].n_os;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0 && v) atomicAdd(&s_total, v);
+  __syncthreads();
+  const unsigned long long total = s_total;
+  for (int j = tid; j < q.n_jobs; j += 1024) {
+    const JobPlan pl = plan_job(q, j, total);
+    q.plan[j] = pl;
+    if (pl.items) atomicAdd(&s_count[pl.bucket], (unsigned)pl.items);
+  }
+  __syncthreads();
+  if (tid < 32) {  // exclusive scan of the buckets, two per lane
+    static_assert(kPlanBuckets == 64, "two buckets per lane");
+    const unsigned a = s_count[2 * lane], b = s_count[2 * lane + 1];
+    unsigned incl = a + b;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const unsigned base = incl - a - b;
+    s_start[2 * lane] = base;
+    s_start[2 * lane + 1] = base + a;
+    q.bucket_start[2 * lane] = base;
+    q.bucket_start[2 * lane + 1] = base + a;
+    if (lane == 31) *q.n_items = (long long)incl <= q.item_cap ? (int)incl : (int)q.item_cap;
+  }
+  if (q.n_jobs > kPlanSmall) return;
+  if (tid < kPlanBuckets) s_count[tid] = 0;  // from here the buckets' cursors
+  __syncthreads();
+  for (int j = tid >> 5; j < q.n_jobs; j += 32) {
+    const JobPlan pl = q.plan[j];
+    if (pl.items == 0) continue;
+    unsigned at = 0;
+    if (lane == 0) at = s_start[pl.bucket] + atomicAdd(&s_count[pl.bucket], (unsigned)pl.items);
+    at = __shfl_sync(0xffffffffu, at, 0);
+    plan_items(q, j, pl, at, lane, 32);
+  }
 }
 
-cudaError_t launch_reset_aux(JobAux* aux, int n, cudaStream_t s) {
-  if (n <= 0) return cudaSuccess;
-  k_reset_aux<<<(n + 255) / 256, 256, 0, s>>>(aux, n);
+__global__ void __launch_bounds__(128) k_plan_write(PlanParams q) {
+  const int j = blockIdx.x;
+  const JobPlan pl = q.plan[j];
+  if (pl.items == 0) return;
+  __shared__ unsigned s_pos;
+  if (threadIdx.x == 0)
+    s_pos = q.bucket_start[pl.bucket] + atomicAdd(&q.bucket_cursor[pl.bucket], (unsigned)pl.items);
+  __syncthreads();
+  plan_items(q, j, pl, s_pos, threadIdx.x, 128);
+}
+
+// The run's state on the device to its initial values. One kernel rather than a memset per array: ten
+// operations in a row cost a small batch more than its superimposition; and no copy from the host:
+// a host-to-device copy on the run's stream would queue on a copy engine behind any track upload in
+// flight and hold the run's kernels back.
+__global__ void __launch_bounds__(256) k_reset(const __grid_constant__ ResetParams p) {
+  const int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x, step = (int64_t)gridDim.x * 256;
+  for (int64_t j = i0; j < p.n_jobs; j += step) {
+    JobAux a = {};
+    a.e_min = INT_MAX;
+    a.e_max = INT_MIN;
+    p.aux[j] = a;
+  }
+  for (int64_t i = i0; i < p.n_units; i += step) {
+    p.u_next[i] = 0;
+    p.u_done[i] = 0;
+    p.u_table[i] = ~0u;
+  }
+  for (int64_t i = i0; i < p.n_bins; i += step) p.bins[i] = 0;
+  for (int64_t i = i0; i < p.n_pool; i += step) p.pool[i] = 0;
+  for (int64_t i = i0; i < kPlanScratch / 4; i += step) p.plan[i] = 0;
+  if (i0 < 4) {
+    p.counter[i0] = 0;
+    if (p.err) p.err[i0] = 0;
+    if (p.ex_count) p.ex_count[i0] = 0;
+  }
+  if (p.gkeys) {
+    for (int64_t i = i0; i < p.n_slots; i += step) {
+      p.gkeys[i] = kEmptyKey;
+      p.glo[i] = 0;
+      p.ghi[i] = 0;
+    }
+    for (int64_t i = i0; i < p.n_tables; i += step) p.gcount[i] = 0;
+  }
+}
+
+cudaError_t launch_reset(const ResetParams& p, cudaStream_t s) {
+  int64_t most = p.n_jobs > p.n_units ? p.n_jobs : p.n_units;
+  if (p.n_bins > most) most = p.n_bins;
+  if (p.gkeys && p.n_slots > most) most = p.n_slots;
+  const int64_t blocks = (most + 255) / 256;
+  k_reset<<<(unsigned)(blocks < 1 ? 1 : blocks > 592 ? 592 : blocks), 256, 0, s>>>(p);
   return cudaGetLastError();
 }
 
+int plan_launches(int n_jobs) { return n_jobs <= 0 ? 0 : n_jobs > kPlanSmall ? 2 : 1; }
+
 cudaError_t launch_plan(const PlanParams& q, cudaStream_t s) {
   if (q.n_jobs <= 0) return cudaSuccess;
-  const int blocks = (q.n_jobs + 255) / 256;
-  k_plan_total<<<blocks, 256, 0, s>>>(q);
-  k_plan_size<<<blocks, 256, 0, s>>>(q);
-  k_plan_scan<<<1, 32, 0, s>>>(q);
-  k_plan_write<<<q.n_jobs, 128, 0, s>>>(q);
+  k_plan<<<1, 1024, 0, s>>>(q);
+  if (q.n_jobs > kPlanSmall) k_plan_write<<<q.n_jobs, 128, 0, s>>>(q);
   return cudaGetLastError();
 }
 
