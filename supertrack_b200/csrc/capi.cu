@@ -16,15 +16,16 @@
 
 namespace st {
 cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_flagged,
-                           cudaStream_t s);
+                           bool chained, cudaStream_t s);
 cudaError_t configure_fused();
 bool fused_big_table(int max_nbins, int table_slots);
-cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s);
+cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, bool chained,
+                         cudaStream_t s);
 cudaError_t launch_fp64_probe(double* out, int blocks, int iters, cudaStream_t s);
 cudaError_t launch_unit_wait_probe(int* table, int* error_flags, int* out, long long max_polls,
                                    cudaStream_t s);
 cudaError_t launch_smem_atomic_probe(unsigned long long* out, int blocks, int iters, cudaStream_t s);
-cudaError_t launch_plan(const PlanParams& q, cudaStream_t s);
+cudaError_t launch_plan(const PlanParams& q, bool chained, cudaStream_t s);
 cudaError_t launch_reset(const ResetParams& p, cudaStream_t s);
 int plan_launches(int n_jobs);
 }  // namespace st
@@ -646,15 +647,15 @@ st_status enqueue_run(st_ctx* c, const st::FusedParams& fp, size_t nj, bool want
   ST_CUDA(st::launch_reset(reset_params(c, nj, want_export), c->stream), "reset");
 
   ST_CUDA(cudaEventRecordWithFlags(c->ev[0], c->stream, evf), "event");
-  ST_CUDA(st::launch_prepare(c->cache_pp, c->cache_blocks, c->cache_any_flagged, c->stream), "prepare launch");
-  ST_CUDA(st::launch_plan(c->cache_plan, c->stream), "plan launch");
+  ST_CUDA(st::launch_prepare(c->cache_pp, c->cache_blocks, c->cache_any_flagged, false, c->stream), "prepare launch");
+  ST_CUDA(st::launch_plan(c->cache_plan, c->cache_blocks > 0, c->stream), "plan launch");
   ST_CUDA(cudaEventRecordWithFlags(c->ev[1], c->stream, evf), "event");
   if (c->order_after && !capturing) {
     ST_CUDA(cudaStreamWaitEvent(c->stream, c->order_after, 0), "order after");
     c->order_after = nullptr;
   }
   ST_CUDA(cudaEventRecordWithFlags(c->ev[4], c->stream, evf), "event");
-  ST_CUDA(st::launch_fused(fp, c->cache_max_nbins, c->cache_grid, c->table_slots, c->stream), "fused launch");
+  ST_CUDA(st::launch_fused(fp, c->cache_max_nbins, c->cache_grid, c->table_slots, false, c->stream), "fused launch");
   ST_CUDA(cudaEventRecordWithFlags(c->ev[2], c->stream, evf), "event");
   ST_CUDA(cudaMemcpyAsync(c->h_aux, c->d_aux.p, nj * sizeof(JobAux), cudaMemcpyDeviceToHost, c->stream), "read aux");
   ST_CUDA(cudaMemcpyAsync(c->h_err, c->d_err.p, 16, cudaMemcpyDeviceToHost, c->stream), "read errors");
@@ -691,13 +692,13 @@ st_status enqueue_groups(st_ctx* c, const st::FusedParams& fp, size_t first,
     pp.blk_base = c->cache_blk[j0];
     bool flagged = false;
     for (size_t j = j0; j < j1; ++j) flagged |= c->cache_flagged[j] != 0;
-    ST_CUDA(st::launch_prepare(pp, c->cache_blk[j1] - c->cache_blk[j0], flagged, c->stream), "prepare launch");
+    ST_CUDA(st::launch_prepare(pp, c->cache_blk[j1] - c->cache_blk[j0], flagged, false, c->stream), "prepare launch");
     st::PlanParams q = c->cache_plan;
     q.jobs += j0;
     q.aux += j0;
     q.plan += j0;
     q.n_jobs = (int32_t)(j1 - j0);
-    ST_CUDA(st::launch_plan(q, c->stream), "plan launch");
+    ST_CUDA(st::launch_plan(q, c->cache_blk[j1] > c->cache_blk[j0], c->stream), "plan launch");
     if (g == 0) {
       ST_CUDA(cudaEventRecord(c->ev[1], c->stream), "event");
       ST_CUDA(cudaEventRecord(c->ev[4], c->stream), "event");
@@ -705,7 +706,7 @@ st_status enqueue_groups(st_ctx* c, const st::FusedParams& fp, size_t first,
     st::FusedParams f = fp;
     f.jobs += j0;
     f.aux += j0;
-    ST_CUDA(st::launch_fused(f, c->cache_max_nbins, c->cache_grid, c->table_slots, c->stream), "fused launch");
+    ST_CUDA(st::launch_fused(f, c->cache_max_nbins, c->cache_grid, c->table_slots, false, c->stream), "fused launch");
   }
   ST_CUDA(cudaEventRecord(c->ev[2], c->stream), "event");
   ST_CUDA(cudaMemcpyAsync(c->h_aux, c->d_aux.p, nj * sizeof(JobAux), cudaMemcpyDeviceToHost, c->stream), "read aux");
