@@ -70,10 +70,14 @@ struct Layout {
 constexpr Layout make_layout() {
   Layout L{};
   size_t o = 0;
+  // uploaded by one copy: descriptors, then the edges in use
   L.jobs = o;       o += al(sizeof(st::JobDev));
-  L.aux = o;        o += al(sizeof(st::JobAux));
   L.hists = o;      o += al(sizeof(st::HistDev));
   L.blk_prefix = o; o += al(2 * 8);
+  L.edges = o;      o += al((size_t)(kNaMaxBins + 1) * 8);
+  // read back by one copy
+  L.aux = o;        o += al(sizeof(st::JobAux));
+  L.err = o;        o += al(16);
   L.blk_count = o;  o += al(kNaBlocks * 4);
   L.blk_off = o;    o += al(kNaBlocks * 8);
   L.pg = o;         o += al(kNaMaxDeposits * 8);
@@ -94,8 +98,6 @@ constexpr Layout make_layout() {
   L.plan = o;       o += al(sizeof(st::JobPlan));
   L.plan_misc = o;  o += al(16 + 3 * 4 * st::kPlanBuckets);
   L.counter = o;    o += al(16);
-  L.err = o;        o += al(16);
-  L.edges = o;      o += al((size_t)(kNaMaxBins + 1) * 8);
   L.units = o;      o += al(3 * 4);
   L.total = o;
   return L;
@@ -158,7 +160,9 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   if (desc->zshift < ST_ZSHIFT_PLUS || desc->zshift > ST_ZSHIFT_NONE) return ST_ERR_INVALID_ARGUMENT;
   st::Geometry g;
   if (st::make_geometry(desc->half_length, desc->sphere_diameter, &g) != 0) return ST_ERR_BAD_GEOMETRY;
-  double edges[kNaMaxBins + 1];
+  // what the call uploads, as it lies at the start of the scratch (host stack)
+  alignas(256) unsigned char up[kLayout.edges + sizeof(double) * (kNaMaxBins + 1)];
+  double* const edges = reinterpret_cast<double*>(up + kLayout.edges);
   if (hist_type == ST_HIST_LIN) st::LinSpace(lower, upper, nbins, edges);
   else if (hist_type == ST_HIST_LOG) st::LogSpace(lower, upper, nbins, edges);
   else return ST_ERR_BAD_HISTOGRAM;
@@ -174,11 +178,11 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   const cudaStream_t st_ = (cudaStream_t)stream;
   const Layout& L = kLayout;
 
-  // ---- job, histogram and launch descriptors (host stack), copied into the scratch
+  // ---- job, histogram and launch descriptors, copied into the scratch
   const int64_t n = track->n;
   const int64_t n_pad = std::max<int64_t>(256, (n + 255) / 256 * 256);
-  st::JobDev D;
-  std::memset(&D, 0, sizeof(D));
+  std::memset(up, 0, L.edges);
+  st::JobDev& D = *reinterpret_cast<st::JobDev*>(up + L.jobs);
   D.x = track->x; D.y = track->y; D.z = track->z; D.edep = track->edep;
   D.n = n;
   D.n_pad = n_pad;
@@ -211,8 +215,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   D.inv_cell = 1.0 / D.cell_size;
   st::set_integer_geometry(&D);
 
-  st::HistDev H;
-  std::memset(&H, 0, sizeof(H));
+  st::HistDev& H = *reinterpret_cast<st::HistDev*>(up + L.hists);
   H.edges = (const double*)(base + L.edges);
   H.counts = (unsigned long long*)d_counts;
   H.yfy = d_yfy;
@@ -227,17 +230,17 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
     H.cb = nbins / (edges[nbins] - edges[0]);
   }
   const int64_t n_blocks = (n_pad + st::kPrepSlotsPerBlock - 1) / st::kPrepSlotsPerBlock;
-  const int64_t blk[2] = {0, n_blocks};
+  reinterpret_cast<int64_t*>(up + L.blk_prefix)[1] = n_blocks;  // prefix {0, n_blocks}
 
 #define NA_CUDA(call)                                        \
   do {                                                       \
     if ((call) != cudaSuccess) { cudaGetLastError(); return ST_ERR_CUDA; } \
   } while (0)
 
-  NA_CUDA(cudaMemcpyAsync(base + L.jobs, &D, sizeof(D), cudaMemcpyHostToDevice, st_));
-  NA_CUDA(cudaMemcpyAsync(base + L.hists, &H, sizeof(H), cudaMemcpyHostToDevice, st_));
-  NA_CUDA(cudaMemcpyAsync(base + L.blk_prefix, blk, sizeof(blk), cudaMemcpyHostToDevice, st_));
-  NA_CUDA(cudaMemcpyAsync(base + L.edges, edges, (size_t)(nbins + 1) * 8, cudaMemcpyHostToDevice, st_));
+  // one copy each way: every copy between pageable memory and the device is a round trip of the
+  // host (the smallest call 91 us with six copies, 74 us with two)
+  NA_CUDA(cudaMemcpyAsync(base + L.jobs, up + L.jobs, L.edges + (size_t)(nbins + 1) * 8 - L.jobs,
+                          cudaMemcpyHostToDevice, st_));
   // Spill tables: as many as the scratch holds of the size that this track needs (its deposits
   // twice, as in the regular path), one per CTA and at most the pool's 32. (Sixteen CTAs instead
   // of four for a track of 4,000 deposits, its items sized for them, and one reset kernel in place
@@ -342,12 +345,12 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   NA_CUDA(st::launch_fused(fp, nbins, grid, 0, true, st_));
 
   // ---- status: job counters and device error flags (host stack destinations)
-  st::JobAux out;
-  int errflags[4] = {0, 0, 0, 0};
-  NA_CUDA(cudaMemcpyAsync(&out, base + L.aux, sizeof(out), cudaMemcpyDeviceToHost, st_));
-  NA_CUDA(cudaMemcpyAsync(errflags, base + L.err, sizeof(errflags), cudaMemcpyDeviceToHost, st_));
+  alignas(256) unsigned char down[kLayout.err + 16 - kLayout.aux];
+  NA_CUDA(cudaMemcpyAsync(down, base + L.aux, sizeof(down), cudaMemcpyDeviceToHost, st_));
   NA_CUDA(cudaStreamSynchronize(st_));
 #undef NA_CUDA
+  const st::JobAux& out = *reinterpret_cast<const st::JobAux*>(down);
+  const int* const errflags = reinterpret_cast<const int*>(down + (L.err - L.aux));
   if (stats_out) {
     stats_out->hits = out.hits;
     stats_out->spheres = out.spheres;
