@@ -1,0 +1,63 @@
+// The kernels of planning.cuh on the host (cta_emulator.h), as a library for test_planning_on_cpu.py.
+#include "cta_emulator.h"
+// (after the emulator's intrinsics)
+#include "../supertrack_b200/csrc/planning.cuh"
+
+#include <cstring>
+
+namespace {
+std::vector<int> warps(int n, const int32_t* order) { return std::vector<int>(order, order + n); }
+}  // namespace
+
+extern "C" {
+
+// Plans a batch of unlayered jobs (kept deposits and oversamples of each) as the library does;
+// items: 24 bytes per entry as {job, os_begin, os_count, unit, win_begin, win_end}. Returns the
+// number of items that k_plan publishes.
+int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, int grid, int64_t item_cost,
+               int share_divisor, int64_t item_cap, const int32_t* order, int32_t* items_out) {
+  std::vector<st::JobDev> jobs(n_jobs);
+  std::vector<st::JobAux> aux(n_jobs);
+  std::vector<st::JobPlan> plan(n_jobs);
+  std::vector<st::WorkItem> items(item_cap);
+  std::memset(items.data(), 0xFF, items.size() * sizeof(st::WorkItem));
+  for (int j = 0; j < n_jobs; ++j) {
+    std::memset(&jobs[j], 0, sizeof(st::JobDev));
+    std::memset(&aux[j], 0, sizeof(st::JobAux));
+    jobs[j].n = kept[j];
+    jobs[j].n_os = n_os[j];
+    aux[j].kept = kept[j];
+  }
+  unsigned start[st::kPlanBuckets] = {}, cursor[st::kPlanBuckets] = {}, unit = 0;
+  int n_items = 0;
+  st::PlanParams q;
+  std::memset(&q, 0, sizeof(q));
+  q.jobs = jobs.data();
+  q.aux = aux.data();
+  q.n_jobs = n_jobs;
+  q.chunk_windows = 4;
+  q.max_helpers = 32;
+  q.grid = grid;
+  q.item_cost = item_cost;
+  q.share_divisor = share_divisor;
+  q.min_chunks = 4;
+  q.bucket_start = start;
+  q.bucket_cursor = cursor;
+  q.unit_counter = &unit;
+  q.plan = plan.data();
+  q.items = items.data();
+  q.n_items = &n_items;
+  q.item_cap = item_cap;
+  emu::run_cta(1024, dim3(1), 0, warps(32, order), [&] { st::k_plan(q); });
+  if (n_jobs > st::kPlanSmall)
+    for (int j = 0; j < n_jobs; ++j)
+      emu::run_cta(128, dim3(n_jobs), j, warps(4, order + 32), [&] { st::k_plan_write(q); });
+  for (int64_t i = 0; i < item_cap; ++i) {
+    const st::WorkItem& w = items[i];
+    const int32_t v[6] = {w.job, w.os_begin, w.os_count, w.unit, w.win_begin, w.win_end};
+    std::memcpy(items_out + 6 * i, v, sizeof(v));
+  }
+  return n_items;
+}
+
+}  // extern "C"
