@@ -108,6 +108,7 @@ struct HistHost {
   int32_t type = 0, nbins = 0;
   float lower = 0, upper = 0;
   std::vector<double> edges;
+  int32_t keep_bits = 0;  // st::keep_bits of the edges
   int64_t off = 0;        // first bin in the context's count/yfy arenas
   int64_t eoff = 0;       // first edge in the context's edge arena
 };
@@ -422,6 +423,8 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
     hd[h].nbins = c->hists[h].nbins;
     const std::vector<double>& e = c->hists[h].edges;
     const double lo = e.front(), hi = e.back();
+    hd[h].keep_bits = c->hists[h].keep_bits;
+    hd[h].reserved = 0;
     if (c->hists[h].type == ST_HIST_LOG && lo > 0) {
       hd[h].mode = 1;
       hd[h].ca = std::log2(lo);
@@ -1311,6 +1314,7 @@ st_status st_hist_create(st_ctx* c, int32_t type, int32_t nbins, float lower, fl
   if (!c || !hist_id) return ST_ERR_INVALID_ARGUMENT;
   HistHost h;
   if (!st::MakeEdges(type, nbins, lower, upper, &h.edges)) return ST_ERR_BAD_HISTOGRAM;
+  h.keep_bits = st::keep_bits(h.edges.data(), nbins);
   h.type = type; h.nbins = nbins; h.lower = lower; h.upper = upper;
   cudaSetDevice(c->device);
   h.off = c->h_bins;

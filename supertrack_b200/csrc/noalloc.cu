@@ -220,6 +220,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   H.counts = (unsigned long long*)d_counts;
   H.yfy = d_yfy;
   H.nbins = nbins;
+  H.keep_bits = st::keep_bits(edges, nbins);
   if (hist_type == ST_HIST_LOG && edges[0] > 0) {
     H.mode = 1;
     H.ca = std::log2(edges[0]);

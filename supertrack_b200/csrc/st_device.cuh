@@ -22,6 +22,7 @@
 #include <math.h>
 #include <stdint.h>
 #include <cmath>
+#include <cstring>
 #include "st_core.cuh"
 
 namespace st {
@@ -158,7 +159,36 @@ struct HistDev {
   int32_t nbins;
   int32_t mode;                   // bin guess: 0 linear in y, 1 linear in log2(y)
   double ca, cb;                  // guess = (y - ca) * cb  or  (log2(y) - ca) * cb
+  int32_t keep_bits;              // a CTA keeps the histogram for 2^keep_bits deposit*oversamples
+  int32_t reserved;
 };
+
+// A CTA's copy of a histogram holds the y*f(y) sum of a bin as a signed 128-bit integer in units of
+// the lower edge's last place. A y of 2^up times the edge or more (up: the difference of the
+// exponents) has 53 + up bits and 2^k of them have 53 + up + k, which must stay below 127: kSumBits
+// bits are left for up and k. The copy is kept for at most 2^31 deposit*oversamples (32-bit counts),
+// fewer if the widest bin needs the room, down to the 2^18 of one large work item; a y that is too
+// far above its edge even then is added to HBM as a double (sum_span).
+constexpr int kSumBits = 126 - 53;
+inline int keep_bits(const double* edges, int nbins) {
+  int span = 0;
+  for (int b = 0; b < nbins; ++b) {  // (a call without allocation passes here: bits, not ilogb)
+    int64_t lo, hi;
+    std::memcpy(&lo, &edges[b], 8);
+    std::memcpy(&hi, &edges[b + 1], 8);
+    const int e = (int)(lo >> 52), s = (int)(hi >> 52) - e;
+    span = e > 0 && s > span ? s : span;  // (lower edges that are positive normal numbers)
+  }
+  const int k = kSumBits - span;
+  return k < 18 ? 18 : (k > 31 ? 31 : k);
+}
+
+// Largest difference of exponents between a y and its bin's lower edge at which the 128-bit sum
+// takes it, in a copy kept for 2^keep_bits deposit*oversamples or for one item of more (`work`).
+ST_HD int sum_span(int keep_bits, long long work) {
+  const int w = work > 1 ? 64 - clz64((uint64_t)(work - 1)) : 0;  // work <= 2^w
+  return kSumBits - (w > keep_bits ? w : keep_bits);
+}
 
 // One unit of work for the persistent kernel: a contiguous block of oversamples of one job.
 struct WorkItem {

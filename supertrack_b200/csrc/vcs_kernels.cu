@@ -758,6 +758,7 @@ struct CtaState {
   int logn;         // records in the spill log of this oversample
   int table;        // spill table that the CTA holds for its private items (-1: none)
   long long hist_work;  // deposit*oversamples in the shared-memory histogram
+  int hist_span;      // its sum_span
   double sx, sy;      // shift of the current oversample, and in lattice units plus half a cell
   int cx, cy;
 };
@@ -854,6 +855,7 @@ struct BinContext {
   double ca, cb;          // candidate bin = (y - ca) * cb, or (log2 y - ca) * cb
   int E0;
   int job;
+  int span;               // sum_span of the shared-memory histogram
   double scale;           // 2^E0, or 0 when E0 is near the ends of the exponent range
 };
 
@@ -922,11 +924,12 @@ __device__ __forceinline__ void bin_sphere(const BinRegs& R, const BinContext& B
       // in the low word instead.
       const uint64_t eb = (uint64_t)__double_as_longlong(e0);
       if ((int64_t)eb > 0 && (eb >> 52) != 0) {
-        uint64_t lo, hi = 0;
+        uint64_t lo = 0, hi = 0;
         const uint64_t yb = (uint64_t)__double_as_longlong(y);
         const int up = (int)(yb >> 52) - (int)(eb >> 52);  // y >= edge_b: not negative
         if (up < 12) lo = ((yb & 0x000FFFFFFFFFFFFFull) | 0x0010000000000000ull) << up;
-        else to_fixed(y, (int)(eb >> 52) - 1075, &lo, &hi);
+        else if (up <= B.span) to_fixed(y, (int)(eb >> 52) - 1075, &lo, &hi);
+        else atomicAdd(&B.gyfy[b], y);  // the copy's 128 bits could not hold the sum
         unsigned int* w = reinterpret_cast<unsigned int*>(&B.hylo[c]);
         smem_acc_add(w, w + 1, &B.hyhi[c], lo, hi);
       } else {
@@ -1486,6 +1489,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     cs.edges_hist = -1;
     cs.table = -1;
     cs.hist_work = 0;
+    cs.hist_span = 0;
   }
   cudaGridDependencySynchronize();  // (launch_chained: nothing above reads global memory)
   __syncthreads();
@@ -1520,10 +1524,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
 
     // the histogram in shared memory: edges and sums stay while consecutive items use the same
     // one (each item fills a bin by at most its own deposit*oversamples: they are added to HBM
-    // before the 32-bit counts could wrap). 64 short tracks on one 3,000-bin spectrum: fused
+    // before the 32-bit counts or the 128-bit sums could wrap, see keep_bits). 64 short tracks on one 3,000-bin spectrum: fused
     // 0.108 ms with a flush per item, 0.089 ms without.
     const long long work = A.kept * W.os_count;
-    const bool full = hist_work + work > (1ll << 31);
+    const bool full = hist_work + work > (1ll << H.keep_bits);
     if (smem_hist && (cached_hist != F.J.hist || full)) {
       if (cached_hist >= 0) {
         flush_histogram<THREADS>(P.hists[cached_hist], HB, sedges, hcount, hylo, hyhi);
@@ -1534,6 +1538,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
       if (tid == 0) {
         cs.edges_hist = F.J.hist;
         cs.hist_work = 0;
+        cs.hist_span = sum_span(H.keep_bits, work);
       }
     }
 
@@ -1549,6 +1554,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
       sB.E0 = E0;
       sB.scale = E0 > -960 && E0 < 900 ? __longlong_as_double((long long)(E0 + 1023) << 52) : 0.0;
       sB.job = W.job;
+      sB.span = cs.hist_span;
       sB.hcount = smem_hist ? hcount : nullptr;
       sB.hylo = smem_hist ? hylo : nullptr;
       sB.hyhi = smem_hist ? hyhi : nullptr;

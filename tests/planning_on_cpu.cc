@@ -1,4 +1,5 @@
-// The kernels of planning.cuh on the host (cta_emulator.h), as a library for test_planning_on_cpu.py.
+// The kernels of planning.cuh on the host (cta_emulator.h) and host functions of st_device.cuh, as a
+// library for test_planning_on_cpu.py.
 #include "cta_emulator.h"
 // (after the emulator's intrinsics)
 #include "../supertrack_b200/csrc/planning.cuh"
@@ -59,5 +60,8 @@ int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, int grid, i
   }
   return n_items;
 }
+
+int keep_bits(const double* edges, int nbins) { return st::keep_bits(edges, nbins); }
+int sum_span(int keep_bits, int64_t work) { return st::sum_span(keep_bits, work); }
 
 }  // extern "C"

@@ -8,6 +8,8 @@ import subprocess
 import numpy as np
 import pytest
 
+from supertrack_b200 import _capi
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 
 
@@ -69,3 +71,32 @@ def test_plan_covers_every_oversample_once(lib, batch, order):
     # longest first, to within a factor of two and the padding to whole tiles
     assert all(a * 4 + 1024 >= b for a, b in zip(cost, cost[1:]))
     assert np.all(items[n:] == -1)
+
+
+@pytest.mark.parametrize("ratio_bits", [0, 1, 11, 31, 41, 42, 43, 54, 55, 56, 57, 73, 74, 100])
+@pytest.mark.parametrize("lower", [1e-30, 0.01, 3.0])
+@pytest.mark.parametrize("work", [1, 2048, 1 << 18, (1 << 18) + 1, 4_000_000, 1 << 33])
+def test_kept_sums_stay_below_128_bits(lib, ratio_bits, lower, work):
+    """The y*f(y) sum of a bin in shared memory, at the most spheres and the largest y that are
+    added to it between two flushes, comes back from its 128-bit form as it is."""
+    lower = float(np.float32(lower))
+    edges = np.array([lower, lower * 1.7 * 2.0 ** ratio_bits, lower * 4.0 * 2.0 ** ratio_bits])
+    bits = lib.keep_bits(_ptr(edges), 2)
+    span = lib.sum_span(bits, C.c_int64(work))
+    assert 18 <= bits <= 31 and span >= 12     # (an offset below 12 is not compared with the span)
+    if ratio_bits <= 40:
+        assert bits == 31
+    spheres = max(work, 1 << bits)
+    for b in range(2):
+        y = np.nextafter(edges[b + 1], 0.0)
+        up = int(np.frexp(y)[1] - np.frexp(edges[b])[1])
+        if up > span:
+            assert up > 55 or work > 1 << 18
+            y, up = float(np.ldexp(2.0 - 2.0 ** -52, int(np.frexp(edges[b])[1]) - 1 + span)), span
+        e0 = int(np.frexp(edges[b])[1]) - 53    # exponent of the lower edge's last place
+        lo, hi = C.c_uint64(), C.c_uint64()
+        _capi.lib().st_to_fixed(float(y), e0, C.byref(lo), C.byref(hi))
+        total = ((hi.value << 64) | lo.value) * spheres
+        assert total < 1 << 127
+        back = _capi.lib().st_from_fixed(total & (2 ** 64 - 1), total >> 64, e0)
+        assert back == float(y) * spheres
