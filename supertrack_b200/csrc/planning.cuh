@@ -1,8 +1,8 @@
 // Device code that decides how a batch is cut: the scan of the prepare blocks' counts with the choice
-// of window mode (k_prep_scan), the window list of a layered job (cut_windows) and the planner of the
-// fused kernel's work items (k_plan, k_plan_write). Integer arithmetic, warp and CTA steps only, no
-// inline assembly: the CPU tests compile this header with the host compiler and run its kernels
-// under other orders of the warps than a GPU happens to take.
+// of window mode (k_prep_scan), the window list of a layered job (cut_windows), the planner of the
+// fused kernel's work items (k_plan, k_plan_write) and when a CTA empties its table (cta_over).
+// Integer arithmetic, warp and CTA steps only, no inline assembly: the CPU tests compile this header
+// with the host compiler and run it under other orders of the warps than a GPU happens to take.
 #pragma once
 #include <limits.h>
 #include "st_device.cuh"
@@ -176,6 +176,14 @@ __device__ __forceinline__ void cut_windows(const PrepareParams& p, const JobDev
     wins[n] = (unsigned long long)kept;
     aux->n_win = n;
   }
+}
+
+// A barrier of the CTA that returns, in every thread, whether a shared count that threads add to on
+// their way to it ends above `limit`. Whoever adds last sees the final count before arriving; a read
+// after a plain barrier would race with the additions of threads that are already past it, and
+// threads could part ways there.
+__device__ __forceinline__ bool cta_over(const int* count, int limit) {
+  return __syncthreads_or(*(const volatile int*)count > limit) != 0;
 }
 
 // Warp tiles of a shared unit's chunk: chunk_windows windows of kWinTiles tiles per warp,

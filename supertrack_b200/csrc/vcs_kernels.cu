@@ -1412,8 +1412,7 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
       sent = __syncthreads_or(sent);
       if (sent && tid == 0) cs.spilled = 1;
     } else if (window_checks && at < end) {
-      __syncthreads();
-      if (cs.tc[0] > P.flush_threshold) {
+      if (cta_over(&cs.tc[0], P.flush_threshold)) {
         if (log_mode) flush_to_log<CAP, THREADS>(T, cs.tc[0], &cs, P, G);
         else flush_to_spill<CAP, THREADS>(T, cs.tc[0], P, G);
         __syncthreads();

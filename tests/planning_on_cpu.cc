@@ -61,6 +61,30 @@ int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, int grid, i
   return n_items;
 }
 
+// Windows of a CTA that adds `per_window` to a count in each and empties it above `limit` (cta_over).
+// Returns how many threads took another branch than thread 0 at some window's end.
+int empty_windows(int windows, int per_window, int limit, const int32_t* order) {
+  static int count;
+  static unsigned long long took[1024];
+  count = 0;
+  emu::run_cta(1024, dim3(1), 0, warps(32, order), [&] {
+    const int tid = threadIdx.x;
+    took[tid] = 0;
+    for (int w = 0; w < windows; ++w) {
+      if (tid < per_window) atomicAdd(&count, 1);
+      if (st::cta_over(&count, limit)) {
+        took[tid] |= 1ull << w;
+        __syncthreads();
+        if (tid == 0) count = 0;
+        __syncthreads();
+      }
+    }
+  });
+  int other = 0;
+  for (int t = 1; t < 1024; ++t) other += took[t] != took[0];
+  return took[0] ? other : -1;
+}
+
 int keep_bits(const double* edges, int nbins) { return st::keep_bits(edges, nbins); }
 int sum_span(int keep_bits, int64_t work) { return st::sum_span(keep_bits, work); }
 

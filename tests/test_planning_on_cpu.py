@@ -73,6 +73,14 @@ def test_plan_covers_every_oversample_once(lib, batch, order):
     assert np.all(items[n:] == -1)
 
 
+@pytest.mark.parametrize("order", sorted(ORDERS))
+@pytest.mark.parametrize("per_window", [1, 33, 700, 1024])
+def test_threads_agree_when_a_table_is_emptied(lib, per_window, order):
+    """Also at a window that ends with the count at, or one above, the limit."""
+    for limit in (2 * per_window, 2 * per_window - 1, 3 * per_window - 1):
+        assert lib.empty_windows(40, per_window, limit, _ptr(_order(order))) == 0
+
+
 @pytest.mark.parametrize("ratio_bits", [0, 1, 11, 31, 41, 42, 43, 54, 55, 56, 57, 73, 74, 100])
 @pytest.mark.parametrize("lower", [1e-30, 0.01, 3.0])
 @pytest.mark.parametrize("work", [1, 2048, 1 << 18, (1 << 18) + 1, 4_000_000, 1 << 33])
