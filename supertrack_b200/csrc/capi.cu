@@ -19,8 +19,7 @@ cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_fl
                            bool chained, cudaStream_t s);
 cudaError_t configure_fused();
 bool fused_big_table(int max_nbins, int table_slots);
-cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, bool chained,
-                         cudaStream_t s);
+cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s);
 cudaError_t launch_fp64_probe(double* out, int blocks, int iters, cudaStream_t s);
 cudaError_t launch_unit_wait_probe(int* table, int* error_flags, int* out, long long max_polls,
                                    cudaStream_t s);
@@ -658,7 +657,7 @@ st_status enqueue_run(st_ctx* c, const st::FusedParams& fp, size_t nj, bool want
     c->order_after = nullptr;
   }
   ST_CUDA(cudaEventRecordWithFlags(c->ev[4], c->stream, evf), "event");
-  ST_CUDA(st::launch_fused(fp, c->cache_max_nbins, c->cache_grid, c->table_slots, false, c->stream), "fused launch");
+  ST_CUDA(st::launch_fused(fp, c->cache_max_nbins, c->cache_grid, c->table_slots, c->stream), "fused launch");
   ST_CUDA(cudaEventRecordWithFlags(c->ev[2], c->stream, evf), "event");
   ST_CUDA(cudaMemcpyAsync(c->h_aux, c->d_aux.p, nj * sizeof(JobAux), cudaMemcpyDeviceToHost, c->stream), "read aux");
   ST_CUDA(cudaMemcpyAsync(c->h_err, c->d_err.p, 16, cudaMemcpyDeviceToHost, c->stream), "read errors");
@@ -709,7 +708,7 @@ st_status enqueue_groups(st_ctx* c, const st::FusedParams& fp, size_t first,
     st::FusedParams f = fp;
     f.jobs += j0;
     f.aux += j0;
-    ST_CUDA(st::launch_fused(f, c->cache_max_nbins, c->cache_grid, c->table_slots, false, c->stream), "fused launch");
+    ST_CUDA(st::launch_fused(f, c->cache_max_nbins, c->cache_grid, c->table_slots, c->stream), "fused launch");
   }
   ST_CUDA(cudaEventRecord(c->ev[2], c->stream), "event");
   ST_CUDA(cudaMemcpyAsync(c->h_aux, c->d_aux.p, nj * sizeof(JobAux), cudaMemcpyDeviceToHost, c->stream), "read aux");

@@ -34,8 +34,7 @@ namespace st {
 cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_flagged,
                            bool chained, cudaStream_t s);
 cudaError_t configure_fused();
-cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, bool chained,
-                         cudaStream_t s);
+cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s);
 cudaError_t launch_plan(const PlanParams& q, bool chained, cudaStream_t s);
 cudaError_t launch_reset(const ResetParams& p, cudaStream_t s);
 }  // namespace st
@@ -343,7 +342,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
 
   NA_CUDA(st::launch_prepare(pp, n_blocks, D.flagged != 0, true, st_));
   NA_CUDA(st::launch_plan(q, n_blocks > 0, st_));
-  NA_CUDA(st::launch_fused(fp, nbins, grid, 0, true, st_));
+  NA_CUDA(st::launch_fused(fp, nbins, grid, 0, st_));
 
   // ---- status: job counters and device error flags (host stack destinations)
   alignas(256) unsigned char down[kLayout.err + 16 - kLayout.aux];

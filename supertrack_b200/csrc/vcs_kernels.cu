@@ -194,8 +194,9 @@ __device__ __forceinline__ uint64_t nbr_key8(const NbrOffsets& o, int c) {
 // True when one of the neighbour cells c0 .. c0 + BATCH - 1 (keys from key_of) holds a deposit
 // of another window. Their first hash slots are loaded together, so a lane has several L2
 // round trips in flight instead of one; a cell whose first slot holds another key continues
-// probing alone. The hash is read-only here (k_prep_write filled it), and the neighbourhoods of
-// a block's deposits overlap, so cached loads serve many probes from L1.
+// probing alone. The neighbourhoods of a block's deposits overlap, so cached loads serve many probes
+// from L1; plain ones, since k_prep_write may still fill the hash when this kernel is launched
+// (the non-coherent path is for what stays as it is while the kernel lives).
 template <int BATCH, typename KeyOf>
 __device__ __forceinline__ bool cells_foreign(const PrepareParams& p, const JobDev& J,
                                               const KeyOf& key_of, int c0, uint32_t win,
@@ -207,7 +208,7 @@ __device__ __forceinline__ bool cells_foreign(const PrepareParams& p, const JobD
 #pragma unroll
   for (int t = 0; t < BATCH; ++t) {
     h[t] = slot_hash(key_of(c0 + t), mask);
-    v[t] = __ldg(reinterpret_cast<const ulonglong2*>(base + h[t]));
+    v[t] = *reinterpret_cast<const ulonglong2*>(base + h[t]);
   }
   bool foreign = false;
 #pragma unroll
@@ -220,7 +221,7 @@ __device__ __forceinline__ bool cells_foreign(const PrepareParams& p, const JobD
 #pragma unroll 1
       for (uint32_t probe = 1; probe < J.cell_cap; ++probe) {
         hh = (hh + 1) & mask;
-        const ulonglong2 w = __ldg(reinterpret_cast<const ulonglong2*>(base + hh));
+        const ulonglong2 w = *reinterpret_cast<const ulonglong2*>(base + hh);
         if (w.x == key) {
           foreign |= slot_foreign(w, win, shift);
           break;
@@ -698,7 +699,9 @@ __device__ __forceinline__ bool gtable_add(uint64_t* gk, unsigned long long* glo
 }
 
 // Four consecutive 8-byte records (32 bytes, 32-byte aligned: a lane's deposits of a tile) with one
-// 256-bit read-only load.
+// 256-bit read-only load. (k_fused reads all its records through the non-coherent path, so it is never
+// launched chained: they have to stay as they are from its start on. Plain loads, which would allow
+// it, cost the 2,048-track batch 27.2 -> 29.7 ms; the link they would save is about 1 us.)
 __device__ __forceinline__ void ldg_records(const int2* p, unsigned long long* v) {
   asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];"
       : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3])
@@ -1490,7 +1493,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     cs.hist_work = 0;
     cs.hist_span = 0;
   }
-  cudaGridDependencySynchronize();  // (launch_chained: nothing above reads global memory)
   __syncthreads();
 
   for (;;) {
@@ -1742,12 +1744,11 @@ __global__ void __launch_bounds__(256) k_reset(const __grid_constant__ ResetPara
 // allocation 100 / 91 us, one proton track of 19,997 deposits 183 / 168 us, 16 short tracks one at a
 // time 1.68 / 1.56 ms; runs replayed as graphs and large batches stay as they are.
 template <typename P>
-static void launch_chained(void (*kernel)(P), unsigned blocks, unsigned threads, size_t smem,
-                           cudaStream_t s, bool chained, const P& p) {
+static void launch_chained(void (*kernel)(P), unsigned blocks, unsigned threads, cudaStream_t s,
+                           bool chained, const P& p) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(blocks);
   cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr = {};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1770,8 +1771,8 @@ int plan_launches(int n_jobs) { return n_jobs <= 0 ? 0 : n_jobs > kPlanSmall ? 2
 
 cudaError_t launch_plan(const PlanParams& q, bool chained, cudaStream_t s) {
   if (q.n_jobs <= 0) return cudaSuccess;
-  launch_chained(k_plan, 1u, 1024u, 0, s, chained, q);
-  if (q.n_jobs > kPlanSmall) launch_chained(k_plan_write, (unsigned)q.n_jobs, 128u, 0, s, true, q);
+  launch_chained(k_plan, 1u, 1024u, s, chained, q);
+  if (q.n_jobs > kPlanSmall) launch_chained(k_plan_write, (unsigned)q.n_jobs, 128u, s, true, q);
   return cudaGetLastError();
 }
 
@@ -1859,12 +1860,12 @@ cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_fl
                            bool chained, cudaStream_t s) {
   if (n_blocks <= 0) return cudaSuccess;
   const unsigned blocks = (unsigned)n_blocks, jobs = (unsigned)p.n_jobs;
-  launch_chained(k_prep_count, blocks, kPrepThreads, 0, s, chained, p);
-  launch_chained(k_prep_scan, jobs, 1024, 0, s, true, p);
-  if (any_flagged) launch_chained(k_prep_cells, 592, kPrepThreads, 0, s, true, p);
-  launch_chained(k_prep_write, blocks, kPrepThreads, 0, s, true, p);
-  launch_chained(k_prep_pad, jobs, kWarpTile, 0, s, true, p);
-  if (any_flagged) launch_chained(k_prep_flag, blocks, kPrepThreads, 0, s, true, p);
+  launch_chained(k_prep_count, blocks, kPrepThreads, s, chained, p);
+  launch_chained(k_prep_scan, jobs, 1024, s, true, p);
+  if (any_flagged) launch_chained(k_prep_cells, 592, kPrepThreads, s, true, p);
+  launch_chained(k_prep_write, blocks, kPrepThreads, s, true, p);
+  launch_chained(k_prep_pad, jobs, kWarpTile, s, true, p);
+  if (any_flagged) launch_chained(k_prep_flag, blocks, kPrepThreads, s, true, p);
   return cudaGetLastError();
 }
 
@@ -1885,22 +1886,20 @@ cudaError_t configure_fused() {
 }
 
 template <bool F32>
-static void launch_fused_form(const FusedParams& p, int grid, bool big_table, bool chained,
-                              cudaStream_t s) {
+static void launch_fused_form(const FusedParams& p, int grid, bool big_table, cudaStream_t s) {
   if (big_table)
-    launch_chained(k_fused<8192, kFusedThreads, F32>, (unsigned)grid, kFusedThreads,
-                   fused_smem_bytes(8192, kSmallHistBins), s, chained, p);
+    k_fused<8192, kFusedThreads, F32>
+        <<<grid, kFusedThreads, fused_smem_bytes(8192, kSmallHistBins), s>>>(p);
   else
-    launch_chained(k_fused<4096, kFusedThreads, F32>, (unsigned)grid, kFusedThreads,
-                   fused_smem_bytes(4096, kBigHistBins), s, chained, p);
+    k_fused<4096, kFusedThreads, F32>
+        <<<grid, kFusedThreads, fused_smem_bytes(4096, kBigHistBins), s>>>(p);
 }
 
 // Picks the kernel shape: the 8192-slot sphere table when the largest histogram of the batch
 // fits the remaining shared memory (and table_slots does not ask for 4096), else 4096 slots with
 // room for 4096 bins; fills P.smem_hist_bins and P.flush_threshold. P.fp32 picks the FP32
 // geometry form.
-cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, bool chained,
-                         cudaStream_t s) {
+cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s) {
   if (grid <= 0) return cudaSuccess;
   const bool big_table = fused_big_table(max_nbins, table_slots);
   if (big_table) {
@@ -1910,8 +1909,8 @@ cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots
     p.smem_hist_bins = kBigHistBins;
     p.flush_threshold = 4096 / 2;
   }
-  if (p.fp32) launch_fused_form<true>(p, grid, big_table, chained, s);
-  else launch_fused_form<false>(p, grid, big_table, chained, s);
+  if (p.fp32) launch_fused_form<true>(p, grid, big_table, s);
+  else launch_fused_form<false>(p, grid, big_table, s);
   return cudaGetLastError();
 }
 
