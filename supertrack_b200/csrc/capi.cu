@@ -206,7 +206,7 @@ struct st_ctx {
   int64_t cache_item_cap = 0;
   st::PlanParams cache_plan{};
   int chunk_windows = 4;      // windows (8192 deposits each) per chunk of a shared unit
-  int max_helpers = 32;       // helper items per shared unit
+  int max_helpers = st::kMaxHelpers;       // helper items per shared unit
   int64_t spill_budget = 0;   // bytes for the spill tables; 0: 30% of free memory (or the full
                               // grid's tables if they leave 16 GB free), at most 48 GB
   int share_divisor = 8;      // shared units: kept > batch units / (share_divisor * grid) ...
@@ -373,8 +373,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
     D.shift_track = J.desc.shift_track ? 1 : 0;
     D.hist = J.desc.hist_id;
     // boundary flags pay off for multi-window jobs on fine lattices with several oversamples
-    D.flagged = (J.track.n > 2 * st::kCtaTile && J.desc.n_oversamples >= 4 &&
-                 D.N >= 128 && D.N < (1u << (st::kCellBits - 2))) ? 1 : 0;
+    D.flagged = st::job_flagged(J.track.n, J.desc.n_oversamples, D.N) ? 1 : 0;
     D.cell_cap = 0;
     D.cell_off = 0;
     // flag cells: two hits of one sphere are within d of each other; in the FP32 form within d
@@ -399,7 +398,6 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
       cells_total += D.cell_cap;
       any_flagged = true;
     }
-    // z bins: one per lattice layer, or per 2^k layers on a lattice of more than kMaxBins
     D.bin_off = bins_total;
     D.win_off = wins_total;
     D.n_bins = 0;
@@ -407,8 +405,8 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
     D.layers = (D.flagged && c->sort_deposits >= 1 && J.track.n < ((int64_t)1 << 31)) ? 1 : 0;
     D.reserved = 0;
     if (D.layers) {
-      while (((D.N - 1) >> D.bin_shift) >= (uint32_t)st::kMaxBins) ++D.bin_shift;
-      D.n_bins = (int32_t)((D.N - 1) >> D.bin_shift) + 1;
+      D.bin_shift = st::bin_shift(D.N);
+      D.n_bins = st::bin_count(D.N);
       bins_total += D.n_bins;
       wins_total += st::window_cap(J.track.n, (int64_t)win_tiles * st::kWarpTile);
     }

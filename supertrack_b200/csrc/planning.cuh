@@ -251,7 +251,6 @@ __device__ __forceinline__ JobPlan plan_job(const PlanParams& q, int j, unsigned
       } else {
         long long b = ic / kept;
         b = b < 1 ? 1 : (b > nos ? nos : b);
-        pl.blk_win = (int)n_win;
         pl.blk_os = (int)b;
         pl.items = (int)((nos + b - 1) / b);
         pl.bucket = cost_bucket(kept * b);
@@ -284,17 +283,11 @@ __device__ __forceinline__ void plan_items(const PlanParams& q, int j, const Job
     if (pos >= q.item_cap) break;
     WorkItem w;
     w.job = j;
-    w.win_begin = 0;
-    w.win_end = 0;
     if (pl.blk_win > 0) {
-      const int n_win = q.aux[j].n_win;
-      const int parts = (n_win + pl.blk_win - 1) / pl.blk_win;
-      const int o = k / parts, part = k % parts;
-      w.os_begin = o * pl.blk_os;
-      w.os_count = (w.os_begin + pl.blk_os <= nos) ? pl.blk_os : nos - w.os_begin;
-      w.unit = -1;
-      w.win_begin = part * pl.blk_win;
-      w.win_end = min(w.win_begin + pl.blk_win, n_win);
+      const int parts = (q.aux[j].n_win + pl.blk_win - 1) / pl.blk_win;
+      w.os_begin = k / parts;
+      w.os_count = -pl.blk_win;
+      w.unit = -1 - k % parts;
     } else if (pl.unit_base >= 0) {
       const int u = k / pl.blk_os;
       w.os_begin = u;

@@ -33,7 +33,7 @@
 #include <vector>
 
 #include "../../include/supertrack_b200.h"
-#include "st_core.cuh"
+#include "st_device.cuh"
 
 namespace {
 
@@ -62,25 +62,17 @@ struct ServedJob {
   int64_t footprint = 0;
 };
 
-int64_t pad256(int64_t n) { return (std::max<int64_t>(n, 1) + 255) / 256 * 256; }
-
 uint64_t pow2_at_least(uint64_t v) {
   uint64_t p = 1;
   while (p < v) p <<= 1;
   return p;
 }
 
-// Device bytes one job holds while its batch is in flight: its track (x, y, z, edep), the
-// prepared records (x, y, dz^2 in FP64 and in lattice units, two fixed-point words, key), the boundary-cell hash and shifted z
-// of window-flagged jobs, its histogram (counts, y*f(y), edges), its job tables and work items.
+int64_t pad256(int64_t n) { return (std::max<int64_t>(n, 1) + 255) / 256 * 256; }
+
+// Device bytes one job holds while its batch is in flight.
 int64_t job_footprint(const st_track_view& t, const st_job_desc& d, int32_t nbins, uint32_t n_lin) {
-  const int64_t n = t.n, np = pad256(n);
-  int64_t b = 32 * n + 60 * np;
-  const bool flagged = n > 2 * 4096 && d.n_oversamples >= 4 && n_lin >= 128 && n_lin < (1u << 19);
-  if (flagged) b += 16 * (int64_t)pow2_at_least(2 * (uint64_t)n) + 8 * np;
-  b += 24 * (int64_t)nbins + 8;
-  b += 512 + 16 * 32 * (int64_t)d.n_oversamples + 12 * (int64_t)d.n_oversamples;
-  return b;
+  return st::job_device_bytes(t.n, d.n_oversamples, n_lin, nbins, st::kMaxHelpers);
 }
 
 struct Slot {

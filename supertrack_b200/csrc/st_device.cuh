@@ -27,6 +27,7 @@
 
 namespace st {
 
+constexpr int64_t kRecordBytes = 8 + 4 + 16 + 8 + 16 + 8;  // PG, PGZ, PXY, PDZ2, PV, PKEY
 constexpr int kDepPerLane = 4;                  // deposits owned by one lane inside a warp tile
 constexpr int kWarpTile = 32 * kDepPerLane;     // deposits per warp tile
 constexpr uint64_t kEmptyKey = ~0ull;           // never a valid sphere key (keys < 2^63)
@@ -132,6 +133,15 @@ constexpr unsigned long long kWinContinues = 1ull << 63;  // window list: the bi
 // deposits, a bin larger than a window ends with a short one, plus the closing entry.
 constexpr int64_t window_cap(int64_t n, int64_t win_deposits) { return 3 * (n / win_deposits) + 8; }
 
+// z bins of a layered job: one per lattice layer, or per 2^bin_shift layers on a lattice of more
+// than kMaxBins.
+inline int bin_shift(uint32_t N) {
+  int s = 0;
+  while (((N - 1) >> s) >= (uint32_t)kMaxBins) ++s;
+  return s;
+}
+inline int bin_count(uint32_t N) { return (int)((N - 1) >> bin_shift(N)) + 1; }
+
 // Per-job values produced on the device.
 struct JobAux {
   int32_t e_min;          // min ulp exponent over nonzero contributions
@@ -190,15 +200,15 @@ ST_HD int sum_span(int keep_bits, long long work) {
   return kSumBits - (w > keep_bits ? w : keep_bits);
 }
 
-// One unit of work for the persistent kernel: a contiguous block of oversamples of one job.
+// One unit of work for the persistent kernel: a contiguous block of oversamples of one job, or part
+// of one oversample. A batch has room for total oversamples * max_helpers of them: 16 bytes.
 struct WorkItem {
   int32_t job;
   int32_t os_begin;
-  int32_t os_count;
-  int32_t unit;       // -1: the CTA does every window of os_begin..+os_count; else a helper of
-                      // shared unit `unit` (one oversample of a large job, split into chunks)
-  int32_t win_begin;  // layered jobs: the windows of each oversample that the item covers
-  int32_t win_end;
+  int32_t os_count;   // negative: part of oversample os_begin of a layered job, -os_count windows
+  int32_t unit;       // >= 0: a helper of shared unit `unit` (one oversample of a large job, split
+                      // into chunks); -1: the CTA does every window of its oversamples; -1 - p:
+                      // part p of the oversample
 };
 
 // One exported sphere: (oversample, key, lineal energy, hit deposits).
@@ -290,13 +300,14 @@ struct PrepareParams {
 };
 
 // Device-side planning of the fused kernel's work items from the kept deposit counts.
+constexpr int kMaxHelpers = 32;  // default of JobPlan's helpers per unit and parts per oversample
 constexpr int kPlanBuckets = 64;
 struct JobPlan {
   int32_t items;
   int32_t bucket;
   int32_t unit_base;   // -1: private items
   int32_t blk_os;      // oversamples per private item, or helpers per unit
-  int32_t blk_win;     // layered jobs: windows per item (0: not layered)
+  int32_t blk_win;     // windows per item of a job whose oversamples are split into parts, else 0
 };
 struct PlanParams {
   const JobDev* jobs;
@@ -358,5 +369,30 @@ constexpr int kWindow = kWinTiles * kCtaTile;         // kept deposits per windo
 // this (context parameter flag_cells_limit).
 constexpr int64_t kFlagCellsLimit = 25000;
 constexpr int kCellBits = 21;                         // bits per axis of a cell key
+
+// A job qualifies for windows (JobDev::flagged): several of them, on a fine lattice, for several
+// oversamples.
+inline bool job_flagged(int64_t n, int64_t n_os, uint32_t N) {
+  return n > 2 * kCtaTile && n_os >= 4 && N >= 128 && N < (1u << (kCellBits - 2));
+}
+
+// Device bytes that one job of a batch takes in a context's arrays: its track (x, y, z, edep), the
+// prepared records, the cell hash and shifted z, z bins and window list of a job that qualifies for
+// windows, its tables, prepare blocks, work items and units, and one histogram of its own. The
+// server admits jobs by it, so it must not be less than what build_tables allocates per job.
+inline int64_t job_device_bytes(int64_t n, int64_t n_os, uint32_t N, int nbins, int max_helpers) {
+  const int64_t n_pad = ((n > 1 ? n : 1) + 255) / 256 * 256;
+  const int64_t blocks = (n_pad + kPrepSlotsPerBlock - 1) / kPrepSlotsPerBlock;
+  int64_t b = 32 * n + kRecordBytes * n_pad;
+  if (job_flagged(n, n_os, N)) {
+    int64_t cells = 1;
+    while (cells < 2 * n) cells <<= 1;
+    b += cells * (int64_t)sizeof(CellSlot) + 8 * n_pad;
+    b += 4 * (int64_t)bin_count(N) + 8 * window_cap(n, kCtaTile);
+  }
+  b += (int64_t)(sizeof(JobDev) + sizeof(JobAux) + sizeof(JobPlan) + sizeof(HistDev)) + 8 + 16 * blocks;
+  b += n_os * (max_helpers * (int64_t)sizeof(WorkItem) + 12);
+  return b + 16 * (int64_t)nbins + 8 * ((int64_t)nbins + 1);
+}
 
 }  // namespace st

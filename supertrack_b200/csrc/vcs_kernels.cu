@@ -1527,7 +1527,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
     // one (each item fills a bin by at most its own deposit*oversamples: they are added to HBM
     // before the 32-bit counts or the 128-bit sums could wrap, see keep_bits). 64 short tracks on one 3,000-bin spectrum: fused
     // 0.108 ms with a flush per item, 0.089 ms without.
-    const long long work = A.kept * W.os_count;
+    const int n_os = W.os_count < 0 ? 1 : W.os_count;
+    const long long work = A.kept * n_os;
     const bool full = hist_work + work > (1ll << H.keep_bits);
     if (smem_hist && (cached_hist != F.J.hist || full)) {
       if (cached_hist >= 0) {
@@ -1589,15 +1590,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_fused(FusedParams P) {
       int os, t;
       int64_t wb, we;
       if (!shared) {
-        if (private_table < 0 || seg >= W.os_count) break;
+        if (private_table < 0 || seg >= n_os) break;
         os = W.os_begin + seg;
         t = private_table;
         wb = 0;
         we = n_wt;
         if (F.wins) {
           // whole bins: a window that continues a bin belongs to the item that began it
-          wb = W.win_begin;
-          we = W.win_end;
+          wb = W.os_count < 0 ? (int64_t)(-1 - W.unit) * -W.os_count : 0;
+          we = W.os_count < 0 ? min(wb - W.os_count, (int64_t)A.n_win) : (int64_t)A.n_win;
           while (wb < A.n_win && (F.wins[wb] & kWinContinues)) ++wb;
           while (we < A.n_win && (F.wins[we] & kWinContinues)) ++we;
         }

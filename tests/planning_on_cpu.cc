@@ -12,10 +12,10 @@ std::vector<int> warps(int n, const int32_t* order) { return std::vector<int>(or
 
 extern "C" {
 
-// Plans a batch of unlayered jobs (kept deposits and oversamples of each) as the library does;
-// items: 24 bytes per entry as {job, os_begin, os_count, unit, win_begin, win_end}. Returns the
-// number of items that k_plan publishes.
-int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, int grid, int64_t item_cost,
+// Plans a batch of jobs (kept deposits, oversamples and, for layered jobs, windows of each) as the
+// library does; items_out: {job, os_begin, os_count, unit} per entry. Returns the number of items
+// that k_plan publishes.
+int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, const int32_t* n_win, int grid, int64_t item_cost,
                int share_divisor, int64_t item_cap, const int32_t* order, int32_t* items_out) {
   std::vector<st::JobDev> jobs(n_jobs);
   std::vector<st::JobAux> aux(n_jobs);
@@ -28,6 +28,8 @@ int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, int grid, i
     jobs[j].n = kept[j];
     jobs[j].n_os = n_os[j];
     aux[j].kept = kept[j];
+    aux[j].n_win = n_win[j];
+    aux[j].windowed = n_win[j] > 0 ? st::kWinLayers : st::kWinNone;
   }
   unsigned start[st::kPlanBuckets] = {}, cursor[st::kPlanBuckets] = {}, unit = 0;
   int n_items = 0;
@@ -55,8 +57,8 @@ int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, int grid, i
       emu::run_cta(128, dim3(n_jobs), j, warps(4, order + 32), [&] { st::k_plan_write(q); });
   for (int64_t i = 0; i < item_cap; ++i) {
     const st::WorkItem& w = items[i];
-    const int32_t v[6] = {w.job, w.os_begin, w.os_count, w.unit, w.win_begin, w.win_end};
-    std::memcpy(items_out + 6 * i, v, sizeof(v));
+    const int32_t v[4] = {w.job, w.os_begin, w.os_count, w.unit};
+    std::memcpy(items_out + 4 * i, v, sizeof(v));
   }
   return n_items;
 }
@@ -84,6 +86,14 @@ int empty_windows(int windows, int per_window, int limit, const int32_t* order) 
   for (int t = 1; t < 1024; ++t) other += took[t] != took[0];
   return took[0] ? other : -1;
 }
+
+// Sizes of what a context allocates per job, work item, cell slot and kept deposit.
+void sizes(int64_t* out) {
+  const int64_t v[] = {sizeof(st::JobDev), sizeof(st::JobAux), sizeof(st::JobPlan), sizeof(st::HistDev),
+                       sizeof(st::WorkItem), sizeof(st::CellSlot), st::kRecordBytes};
+  std::memcpy(out, v, sizeof(v));
+}
+int64_t window_cap(int64_t n, int64_t win_deposits) { return st::window_cap(n, win_deposits); }
 
 int keep_bits(const double* edges, int nbins) { return st::keep_bits(edges, nbins); }
 int sum_span(int keep_bits, int64_t work) { return st::sum_span(keep_bits, work); }

@@ -57,12 +57,12 @@ def test_plan_covers_every_oversample_once(lib, batch, order):
     kept = np.array([k for k, _ in jobs], dtype=np.int64)
     n_os = np.array([o for _, o in jobs], dtype=np.int32)
     cap = int(n_os.sum()) * 32 + 8
-    items = np.zeros((cap, 6), dtype=np.int32)
-    n = lib.plan_batch(len(jobs), _ptr(kept), _ptr(n_os), 148, C.c_int64(1 << 18), 0,
+    items = np.zeros((cap, 4), dtype=np.int32)
+    n = lib.plan_batch(len(jobs), _ptr(kept), _ptr(n_os), _ptr(np.zeros_like(n_os)), 148, C.c_int64(1 << 18), 0,
                        C.c_int64(cap), _ptr(_order(order)), _ptr(items))
     done = [np.zeros(o, dtype=int) for o in n_os]
     cost = []
-    for job, first, count, unit, _, _ in items[:n]:
+    for job, first, count, unit in items[:n]:
         assert 0 <= job < len(jobs) and unit < 0 and count > 0
         done[job][first:first + count] += 1
         cost.append(int(kept[job]) * int(count))
@@ -71,6 +71,58 @@ def test_plan_covers_every_oversample_once(lib, batch, order):
     # longest first, to within a factor of two and the padding to whole tiles
     assert all(a * 4 + 1024 >= b for a, b in zip(cost, cost[1:]))
     assert np.all(items[n:] == -1)
+
+
+@pytest.mark.parametrize("grid", [1, 4, 148])
+@pytest.mark.parametrize("kept,n_os,n_win", [(20_000, 4, 3), (20_000, 400, 1), (300_007, 10, 74),
+                                            (4_000_000, 4, 1), (4_000_000, 3, 977),
+                                            (4_000_000, 50, 33), (300_000, 7, 2)])
+def test_plan_covers_every_window_once(lib, kept, n_os, n_win, grid):
+    """A layered job's items are whole oversamples, or parts of one that cover all its windows."""
+    cap = n_os * 32
+    items = np.zeros((cap, 4), dtype=np.int32)
+    n = lib.plan_batch(1, _ptr(np.array([kept])), _ptr(np.array([n_os], dtype=np.int32)),
+                       _ptr(np.array([n_win], dtype=np.int32)), grid, C.c_int64(1 << 18), 8,
+                       C.c_int64(cap), _ptr(_order("first warp first")), _ptr(items))
+    done = np.zeros((n_os, n_win), dtype=int)
+    for job, first, count, unit in items[:n]:
+        assert job == 0 and unit < 0
+        if count > 0:
+            assert unit == -1
+            done[first:first + count] += 1
+        else:
+            done[first, -count * (-1 - unit):-count * -unit] += 1
+    assert np.all(done == 1)
+
+
+def test_footprint_charges_what_a_job_allocates(lib):
+    """st_server_job_footprint against the arrays of a context that grow with a job."""
+    size = np.zeros(7, dtype=np.int64)
+    lib.sizes(_ptr(size))
+    job, aux, plan, hist, item, slot, record = [int(v) for v in size]
+    lib.window_cap.restype = C.c_int64
+    for n, d, n_os, nbins in [(1, 10.0, 1, 1), (1000, 10.0, 65_536, 4096), (8192, 2.0, 100, 200),
+                              (8193, 2.0, 100, 200), (8193, 1.0, 4, 200), (20_001, 1.3, 4, 3000),
+                              (1_000_000, 2.0, 100, 500), (4_000_000, 10.0, 50, 3000),
+                              (100_000, 1000.0, 50, 200), (200_000, 30.0, 4, 7)]:
+        hl = 2500.0
+        lattice = int(2 * hl / d)
+        pad, blocks = -(-n // 128) * 128, -(-n // 1024)
+        want = (32 * n + record * pad + job + aux + plan + hist + blocks * (8 + 4 + 4) + 8
+                + n_os * (32 * item + 3 * 4) + 16 * nbins + 8 * (nbins + 1))
+        if n > 8192 and n_os >= 4 and 128 <= lattice < 1 << 19:
+            cells = 1 << (2 * n - 1).bit_length()
+            bins = lattice
+            while bins > 4096:
+                bins = (bins + 1) // 2
+            # cell hash, shifted z, z bins, window list (of windows on the smaller table)
+            want += slot * cells + 8 * pad + 4 * bins + 8 * lib.window_cap(C.c_int64(n), C.c_int64(4096))
+        view, desc, got = _capi.st_track_view(), _capi.st_job_desc(), C.c_int64(0)
+        view.n, view.on_device = n, 1
+        desc.half_length, desc.sphere_diameter, desc.n_oversamples = hl, d, n_os
+        assert _capi.lib().st_server_job_footprint(C.byref(view), C.byref(desc), nbins,
+                                                   C.byref(got)) == 0
+        assert got.value >= want
 
 
 @pytest.mark.parametrize("order", sorted(ORDERS))
