@@ -365,7 +365,7 @@ ST_API st_status st_server_drain(st_server* server, int64_t timeout_ms);
  * sharing the GPU cannot afford that), and frameworks that own all device memory through their
  * own pool leave no room for, or forbid, allocations by their plug-ins. The call allocates
  * nothing: it works in a fixed scratch array compiled into the library
- * (st_noalloc_scratch_bytes() bytes, about 6.9 MB, held by every GPU that loads the library
+ * (st_noalloc_scratch_bytes() bytes, about 5.9 MB, held by every GPU that loads the library
  * until the process exits). Limits: one device-resident track (track->on_device != 0) of at
  * most 16384 deposits, at most 65536 oversamples, a histogram of at most 4096 bins; larger
  * requests return ST_ERR_CAPACITY. d_counts (int64) and d_yfy (float64) are device arrays of

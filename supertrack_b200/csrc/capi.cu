@@ -143,9 +143,9 @@ struct st_ctx {
   std::vector<JobHost> jobs;
 
   DevBuf track_arena;
-  DevBuf pg, pgz, pxy, pdz2, pv, pkey;
+  DevBuf pg, pgz, psrc, pv, pkey;
   DevBuf d_jobs, d_aux, d_hists, d_items, d_blk, d_counter, d_err, d_blk_count, d_blk_off, d_blk_job;
-  DevBuf c_cells, pz;               // cell arena and shifted z of flagged jobs
+  DevBuf c_cells;                   // cell arena of flagged jobs
   DevBuf z_bins, z_wins;            // z bins and window lists of layered jobs
   DevBuf u_next, u_done, u_table, pool;  // shared units and the spill-table pool
   DevBuf d_plan, d_plan_misc;             // planner: per-job plans and scratch counters
@@ -314,11 +314,9 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
       arena_total += J.track.n;
     }
   }
-  const int64_t exact_total = c->precision == 32 ? 0 : prep_total;  // FP64 records
   ST_CUDA(ensure(c->pg, prep_total * 8), "prepared arena");
   ST_CUDA(ensure(c->pgz, prep_total * 4), "prepared arena");
-  ST_CUDA(ensure(c->pxy, exact_total * 16), "prepared arena");
-  ST_CUDA(ensure(c->pdz2, exact_total * 8), "prepared arena");
+  ST_CUDA(ensure(c->psrc, prep_total * 4), "prepared arena");
   ST_CUDA(ensure(c->pv, prep_total * 16), "prepared arena");
   ST_CUDA(ensure(c->pkey, prep_total * 8), "prepared arena");
   ST_CUDA(ensure(c->track_arena, (size_t)arena_total * 32), "track arena");
@@ -459,7 +457,6 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   ST_CUDA(ensure(c->c_cells, (size_t)cells_total * sizeof(st::CellSlot)), "cell arena");
   ST_CUDA(ensure(c->z_bins, (size_t)bins_total * 4), "z bins");
   ST_CUDA(ensure(c->z_wins, (size_t)wins_total * 8), "window lists");
-  ST_CUDA(ensure(c->pz, any_flagged ? (size_t)prep_total * 8 : 16), "shifted z");
   ST_CUDA(ensure(c->d_blk_off, (size_t)blk[nj] * 8), "prepare block offsets");
   ST_CUDA(ensure(c->d_counter, 16), "work counter");
   ST_CUDA(ensure(c->d_err, 16), "error flags");
@@ -537,11 +534,9 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   pp.wins = (unsigned long long*)c->z_wins.p;
   pp.win_tiles = win_tiles;
   pp.any_flags = (int32_t*)((char*)c->d_counter.p + 8);
-  pp.PZ = (double*)c->pz.p;
   pp.PG = (int2*)c->pg.p;
   pp.PGZ = (float*)c->pgz.p;
-  pp.PXY = (double2*)c->pxy.p;
-  pp.PDZ2 = (double*)c->pdz2.p;
+  pp.PSRC = (uint32_t*)c->psrc.p;
   pp.PV = (ulonglong2*)c->pv.p;
   pp.PKEY = (unsigned long long*)c->pkey.p;
   pp.fp32 = c->precision == 32 ? 1 : 0;
@@ -557,7 +552,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   fp.flush_threshold = 1024;
   fp.work_counter = (unsigned int*)c->d_counter.p;
   fp.PG = pp.PG; fp.PGZ = pp.PGZ;
-  fp.PXY = pp.PXY; fp.PDZ2 = pp.PDZ2;
+  fp.PSRC = pp.PSRC;
   fp.PV = pp.PV; fp.PKEY = pp.PKEY;
   fp.gkeys = (uint64_t*)c->g_keys.p;
   fp.glo = (unsigned long long*)c->g_lo.p;
@@ -1080,10 +1075,10 @@ st_status st_ctx_destroy(st_ctx* c) {
   if (!c) return ST_ERR_INVALID_ARGUMENT;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  DevBuf* bufs[] = {&c->track_arena, &c->pg, &c->pgz, &c->pxy, &c->pdz2, &c->pv, &c->pkey,
+  DevBuf* bufs[] = {&c->track_arena, &c->pg, &c->pgz, &c->psrc, &c->pv, &c->pkey,
                     &c->d_jobs, &c->d_aux, &c->d_hists, &c->d_items, &c->d_blk,
                     &c->d_counter, &c->d_err, &c->d_blk_count, &c->d_blk_off, &c->d_blk_job, &c->c_cells,
-                    &c->pz, &c->z_bins, &c->z_wins, &c->u_next, &c->u_done, &c->u_table,
+                    &c->z_bins, &c->z_wins, &c->u_next, &c->u_done, &c->u_table,
                     &c->pool, &c->d_plan, &c->d_plan_misc, &c->g_keys, &c->g_lo, &c->g_hi,
                     &c->g_used, &c->g_count, &c->ex_buf, &c->ex_count, &c->h_counts,
                     &c->h_yfy, &c->h_edges};

@@ -8,7 +8,7 @@
 // of the library image.
 //
 // The scratch below is a file-scope __device__ array: every GPU that loads the library holds it
-// (kScratchBytes, about 6.9 MB) until the process exits. Host code cannot pass the symbol
+// (kScratchBytes, about 5.9 MB) until the process exits. Host code cannot pass the symbol
 // itself to a kernel (on the host it names a host-side stand-in), so the first call on each
 // device, with that device current, resolves its device address with cudaGetSymbolAddress and
 // sets the fused kernel's shared-memory attribute; that first call should therefore come before
@@ -59,7 +59,7 @@ constexpr size_t al(size_t v) { return (v + 255) / 256 * 256; }
 // Byte offsets of every region inside the scratch array.
 struct Layout {
   size_t jobs, aux, hists, blk_prefix, blk_count, blk_off;
-  size_t pg, pgz, pxy, pdz2, pv, pkey, pz;
+  size_t pg, pgz, psrc, pv, pkey;
   size_t cells;
   size_t gkeys, glo, ghi, gused, gcount, pool;
   size_t items, plan, plan_misc, counter, err, edges, units;
@@ -81,11 +81,9 @@ constexpr Layout make_layout() {
   L.blk_off = o;    o += al(kNaBlocks * 8);
   L.pg = o;         o += al(kNaMaxDeposits * 8);
   L.pgz = o;        o += al(kNaMaxDeposits * 4);
-  L.pxy = o;        o += al(kNaMaxDeposits * 16);
-  L.pdz2 = o;       o += al(kNaMaxDeposits * 8);
+  L.psrc = o;       o += al(kNaMaxDeposits * 4);
   L.pv = o;         o += al(kNaMaxDeposits * 16);
   L.pkey = o;       o += al(kNaMaxDeposits * 8);
-  L.pz = o;         o += al(kNaMaxDeposits * 8);
   L.cells = o;      o += al((size_t)kNaCellCap * sizeof(st::CellSlot));
   L.gkeys = o;      o += al((size_t)kNaGrid * kNaTableCap * 8);
   L.glo = o;        o += al((size_t)kNaGrid * kNaTableCap * 8);
@@ -280,11 +278,9 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   pp.cells = (st::CellSlot*)(base + L.cells);
   pp.blk_base = 0;
   pp.any_flags = (int32_t*)(base + L.counter + 8);
-  pp.PZ = (double*)(base + L.pz);
   pp.PG = (int2*)(base + L.pg);
   pp.PGZ = (float*)(base + L.pgz);
-  pp.PXY = (double2*)(base + L.pxy);
-  pp.PDZ2 = (double*)(base + L.pdz2);
+  pp.PSRC = (uint32_t*)(base + L.psrc);
   pp.PV = (ulonglong2*)(base + L.pv);
   pp.PKEY = (unsigned long long*)(base + L.pkey);
   // the regular path's default: window flags only above this many kept deposits (a track here
@@ -324,7 +320,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   fp.n_items = q.n_items;
   fp.work_counter = (unsigned int*)(base + L.counter);
   fp.PG = pp.PG; fp.PGZ = pp.PGZ;
-  fp.PXY = pp.PXY; fp.PDZ2 = pp.PDZ2;
+  fp.PSRC = pp.PSRC;
   fp.PV = pp.PV; fp.PKEY = pp.PKEY;
   fp.gkeys = (uint64_t*)(base + L.gkeys);
   fp.glo = (unsigned long long*)(base + L.glo);

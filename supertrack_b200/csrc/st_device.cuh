@@ -10,8 +10,9 @@
 //                 {x, y}); a lane's four records are one 32-byte load
 //       PGZ     : the squared z distance from the layer's centres in the same units (float); a
 //                 lane's four are one 16-byte load
-//       PXY     : {x, y} as loaded, 16 bytes, and
-//       PDZ2    : (k_z*d - a_z)^2, read only for deposits that PG cannot decide
+//       PSRC    : index of the source deposit in the track, for what is read rarely: deposits that
+//                 PG cannot decide, and boundary flags (4 bytes; a track of 2^32 deposits, 128 GB
+//                 of x, y, z, edep and 160 GB of records, does not fit the device)
 //       PV      : v = edep / ((2/3) d) on the job's fixed-point grid, a 128-bit integer stored
 //                 as one 16-byte {low, high} record (one vector load per hit)
 //       PKEY    : k_z * N*N (the z part of the sphere key); bit 63 flags boundary deposits
@@ -27,7 +28,7 @@
 
 namespace st {
 
-constexpr int64_t kRecordBytes = 8 + 4 + 16 + 8 + 16 + 8;  // PG, PGZ, PXY, PDZ2, PV, PKEY
+constexpr int64_t kRecordBytes = 8 + 4 + 4 + 16 + 8;  // PG, PGZ, PSRC, PV, PKEY
 constexpr int kDepPerLane = 4;                  // deposits owned by one lane inside a warp tile
 constexpr int kWarpTile = 32 * kDepPerLane;     // deposits per warp tile
 constexpr uint64_t kEmptyKey = ~0ull;           // never a valid sphere key (keys < 2^63)
@@ -229,8 +230,7 @@ struct FusedParams {
   unsigned int* work_counter; // next item to claim
   const int2* PG;             // {X, Y} in lattice units (FP32 variant: float2 {x, y})
   const float* PGZ;           // squared z distance, in lattice units (FP32 variant: nm)
-  const double2* PXY;         // {x, y} and
-  const double* PDZ2;         // (k_z d - a_z)^2 in FP64, for deposits that PG cannot decide
+  const uint32_t* PSRC;       // index in the track, for deposits that PG cannot decide
   const ulonglong2* PV;            // contribution on the job's grid: {low, high} 64-bit words
   const unsigned long long* PKEY;  // k_z * N*N, bit 63 = boundary deposit
   // spill tables: gridDim.x tables of gcap slots each
@@ -284,11 +284,9 @@ struct PrepareParams {
   unsigned long long* wins;   // window lists of layered jobs
   int32_t win_tiles;          // warp tiles of a layer window (twice that on dense tracks)
   int32_t* any_flags;         // set when a job of the launch runs with window boundary flags
-  double* PZ;                 // z after the z-origin shift (flagged jobs only)
-  int2* PG;                   // records as in FusedParams; PXY and PDZ2 are not written in the
-  float* PGZ;                 // FP32 variant
-  double2* PXY;
-  double* PDZ2;
+  int2* PG;                   // records as in FusedParams
+  float* PGZ;
+  uint32_t* PSRC;
   ulonglong2* PV;
   unsigned long long* PKEY;
   int32_t fp32;               // 1: records for the FP32 geometry variant
@@ -377,8 +375,7 @@ inline bool job_flagged(int64_t n, int64_t n_os, uint32_t N) {
 }
 
 // Device bytes that one job of a batch takes in a context's arrays: its track (x, y, z, edep), the
-// prepared records, the cell hash and shifted z, z bins and window list of a job that qualifies for
-// windows, its tables, prepare blocks, work items and units, and one histogram of its own. The
+// prepared records, the cell hash, z bins and window list of a job that qualifies for windows, its tables, prepare blocks, work items and units, and one histogram of its own. The
 // server admits jobs by it, so it must not be less than what build_tables allocates per job.
 inline int64_t job_device_bytes(int64_t n, int64_t n_os, uint32_t N, int nbins, int max_helpers) {
   const int64_t n_pad = ((n > 1 ? n : 1) + 255) / 256 * 256;
@@ -387,7 +384,7 @@ inline int64_t job_device_bytes(int64_t n, int64_t n_os, uint32_t N, int nbins, 
   if (job_flagged(n, n_os, N)) {
     int64_t cells = 1;
     while (cells < 2 * n) cells <<= 1;
-    b += cells * (int64_t)sizeof(CellSlot) + 8 * n_pad;
+    b += cells * (int64_t)sizeof(CellSlot);
     b += 4 * (int64_t)bin_count(N) + 8 * window_cap(n, kCtaTile);
   }
   b += (int64_t)(sizeof(JobDev) + sizeof(JobAux) + sizeof(JobPlan) + sizeof(HistDev)) + 8 + 16 * blocks;

@@ -518,15 +518,13 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
         p.PG[dst] = make_int2(__double2int_rn(st_dmul(x[r], J.g_scale)),
                               __double2int_rn(st_dmul(y[r], J.g_scale)));
         p.PGZ[dst] = __double2float_rn(st_dmul(gz, gz));
-        p.PXY[dst] = make_double2(x[r], y[r]);
-        p.PDZ2[dst] = st_dmul(dz, dz);
       }
+      p.PSRC[dst] = (uint32_t)(i0 + r * kPrepThreads + threadIdx.x);
       uint64_t lo, hi;
       to_fixed(__ddiv_rn(e[r], J.denom), E0, &lo, &hi);
       p.PV[dst] = make_ulonglong2(lo, hi);
       p.PKEY[dst] = (uint64_t)(long long)kd * J.N2;
       if (A.windowed == kWinFlags) {
-        p.PZ[dst] = z1[r];
         ckey = cell_key(cell_of(x[r], y[r], z1[r], J.inv_cell), 0, 0, 0);
         cwin = (uint32_t)(k / kWindow);
       }
@@ -574,10 +572,7 @@ __global__ void __launch_bounds__(kWarpTile) k_prep_pad(PrepareParams p) {
   if (p.fp32) {
     reinterpret_cast<float2*>(p.PG)[dst] = make_float2(__int_as_float(0x7FC00000), __int_as_float(0x7FC00000));
   } else {
-    p.PG[dst] = make_int2(INT_MIN, INT_MIN);  // outside the voxel for every shift
-    // (read when the job decides every deposit in FP64)
-    p.PXY[dst] = make_double2(__longlong_as_double(0x7FF8000000000000ll),
-                              __longlong_as_double(0x7FF8000000000000ll));
+    p.PG[dst] = make_int2(INT_MIN, INT_MIN);  // outside the voxel for every shift, without FP64
   }
   p.PGZ[dst] = __int_as_float(0x7F800000);
   p.PV[dst] = make_ulonglong2(0, 0);
@@ -604,17 +599,8 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_flag(PrepareParams p) 
   for (int q = threadIdx.x; q < cnt; q += kPrepThreads) {
     const int64_t k = k0 + q;
     const int64_t dst = prep_slot(J, k);
-    double x, y;
-    if (p.fp32) {  // float-rounded x, y: the FP32 jobs' cell size covers the rounding
-      const float2 xy = reinterpret_cast<const float2*>(p.PG)[dst];
-      x = xy.x;
-      y = xy.y;
-    } else {
-      const double2 xy = p.PXY[dst];
-      x = xy.x;
-      y = xy.y;
-    }
-    const double z = p.PZ[dst];
+    const uint32_t src = p.PSRC[dst];
+    const double x = J.x[src], y = J.y[src], z = st_dadd(J.z[src], J.zsh);
     const uint32_t win = (uint32_t)(k / kWindow);
     bool boundary = false;
     // batches unrolled, so that the neighbour offsets are constants
@@ -1313,23 +1299,39 @@ __device__ __forceinline__ void superimpose(const FusedParams& P, const FusedJob
             kyv[p] = vy;
           }
           if (undecided) {
-            // the reference's arithmetic in FP64, each operation rounded on its own
+            // the reference's arithmetic in FP64, each operation rounded on its own, on the track as
+            // it was submitted. (Copies of x, y and the z part beside the records, 20 bytes more per
+            // deposit, spare a lane the index and a second array: 16 tracks of 1e6 deposits, 2 nm,
+            // 23.4 against 24.0 ms, the uneven 2,048-track batch 27.2 and 27.3.)
 #pragma unroll
             for (int p = 0; p < kDepPerLane; ++p) {
               if (undecided & (1u << p)) {
-                const double2 xy = __ldg(&P.PXY[tb + p]);
-                const double x1 = st_dadd(xy.x, cs.sx), y1 = st_dadd(xy.y, cs.sy);
-                const bool inb = fabs(x1) < J.HL && fabs(y1) < J.HL;
+                // (axis by axis: the loop around has no registers to spare for three at once)
+                const uint32_t src = __ldg(&P.PSRC[tb + p]);
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(J.y + src));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(J.z + src));
+                double c = st_dadd(J.x[src], cs.sx);
+                bool inb = fabs(c) < J.HL;
+                c = st_dsub(c, J.gSO);
+                double k = lattice_index(c, J.d, J.inv_d);
+                const int kx = __double2int_rn(k) << S;
+                c = st_dsub(st_dmul(k, J.d), c);
+                double dist = st_dmul(c, c);
+                c = st_dadd(J.y[src], cs.sy);
+                inb = inb && fabs(c) < J.HL;
+                c = st_dsub(c, J.gSO);
+                k = lattice_index(c, J.d, J.inv_d);
+                const int ky = __double2int_rn(k) << S;
+                c = st_dsub(st_dmul(k, J.d), c);
+                dist = st_dadd(dist, st_dmul(c, c));
+                c = st_dsub(st_dadd(J.z[src], J.zsh), J.gSO);
+                k = lattice_index(c, J.d, J.inv_d);
+                c = st_dsub(st_dmul(k, J.d), c);
+                dist = st_dadd(dist, st_dmul(c, c));
                 boxmask = (boxmask & ~(1u << p)) | ((unsigned)inb << p);
-                if (inb) {
-                  const double ax = st_dsub(x1, J.gSO), ay = st_dsub(y1, J.gSO);
-                  const double kx = lattice_index(ax, J.d, J.inv_d), ky = lattice_index(ay, J.d, J.inv_d);
-                  const double dx = st_dsub(st_dmul(kx, J.d), ax), dy = st_dsub(st_dmul(ky, J.d), ay);
-                  const double dist = st_dadd(st_dadd(st_dmul(dx, dx), st_dmul(dy, dy)), __ldg(&P.PDZ2[tb + p]));
-                  hitmask |= (unsigned)(dist <= J.r2) << p;
-                  kxv[p] = __double2int_rn(kx) << S;
-                  kyv[p] = __double2int_rn(ky) << S;
-                }
+                hitmask |= (unsigned)(inb && dist <= J.r2) << p;
+                kxv[p] = kx;
+                kyv[p] = ky;
               }
             }
           }

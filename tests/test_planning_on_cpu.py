@@ -96,7 +96,9 @@ def test_plan_covers_every_window_once(lib, kept, n_os, n_win, grid):
 
 
 def test_footprint_charges_what_a_job_allocates(lib):
-    """st_server_job_footprint against the arrays of a context that grow with a job."""
+    """st_server_job_footprint against the arrays of a context that grow with a job; and no more
+    than 48 bytes of records per deposit and 8 of a qualifying job's shifted z came to, so that what
+    a budget admitted is still admitted."""
     size = np.zeros(7, dtype=np.int64)
     lib.sizes(_ptr(size))
     job, aux, plan, hist, item, slot, record = [int(v) for v in size]
@@ -115,14 +117,19 @@ def test_footprint_charges_what_a_job_allocates(lib):
             bins = lattice
             while bins > 4096:
                 bins = (bins + 1) // 2
-            # cell hash, shifted z, z bins, window list (of windows on the smaller table)
-            want += slot * cells + 8 * pad + 4 * bins + 8 * lib.window_cap(C.c_int64(n), C.c_int64(4096))
+            # cell hash, z bins, window list (of windows on the smaller table)
+            want += slot * cells + 4 * bins + 8 * lib.window_cap(C.c_int64(n), C.c_int64(4096))
         view, desc, got = _capi.st_track_view(), _capi.st_job_desc(), C.c_int64(0)
         view.n, view.on_device = n, 1
         desc.half_length, desc.sphere_diameter, desc.n_oversamples = hl, d, n_os
         assert _capi.lib().st_server_job_footprint(C.byref(view), C.byref(desc), nbins,
                                                    C.byref(got)) == 0
         assert got.value >= want
+        pad256 = -(-n // 256) * 256
+        flagged = n > 8192 and n_os >= 4 and 128 <= lattice < 1 << 19
+        most = (32 * n + 48 * pad256 + 24 * nbins + 8 + 512 + 524 * n_os
+                + ((16 * (1 << (2 * n - 1).bit_length()) + 8 * pad256) if flagged else 0))
+        assert got.value <= most
 
 
 @pytest.mark.parametrize("order", sorted(ORDERS))
