@@ -143,10 +143,12 @@ struct st_ctx {
   std::vector<JobHost> jobs;
 
   DevBuf track_arena;
-  DevBuf pg, pgz, psrc, pv, pkey;
+  DevBuf prep;                      // prepared records, one arena (a context's first run pays for
+                                    // every allocation)
   DevBuf d_jobs, d_aux, d_hists, d_items, d_blk, d_counter, d_err, d_blk_count, d_blk_off, d_blk_job;
   DevBuf c_cells;                   // cell arena of flagged jobs
-  DevBuf z_bins, z_wins;            // z bins and window lists of layered jobs
+  DevBuf z_lists;                   // window lists, then z bins, of layered jobs
+  uint32_t* z_bins = nullptr;
   DevBuf u_next, u_done, u_table, pool;  // shared units and the spill-table pool
   DevBuf d_plan, d_plan_misc;             // planner: per-job plans and scratch counters
   DevBuf g_keys, g_lo, g_hi, g_used, g_count;
@@ -314,11 +316,9 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
       arena_total += J.track.n;
     }
   }
-  ST_CUDA(ensure(c->pg, prep_total * 8), "prepared arena");
-  ST_CUDA(ensure(c->pgz, prep_total * 4), "prepared arena");
-  ST_CUDA(ensure(c->psrc, prep_total * 4), "prepared arena");
-  ST_CUDA(ensure(c->pv, prep_total * 16), "prepared arena");
-  ST_CUDA(ensure(c->pkey, prep_total * 8), "prepared arena");
+  // whole tiles of 128 deposits: every array of records starts on a 256-byte boundary
+  static_assert(st::kWarpTile * 4 % 256 == 0, "the smallest record is 4 bytes");
+  ST_CUDA(ensure(c->prep, (size_t)prep_total * st::kRecordBytes), "prepared arena");
   ST_CUDA(ensure(c->track_arena, (size_t)arena_total * 32), "track arena");
   double* arena = (double*)c->track_arena.p;
 
@@ -455,8 +455,8 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   ST_CUDA(ensure(c->d_blk_count, (size_t)blk[nj] * 4), "prepare block counts");
   ST_CUDA(ensure(c->d_blk_job, (size_t)std::max<int64_t>(1, blk[nj]) * 4), "prepare block jobs");
   ST_CUDA(ensure(c->c_cells, (size_t)cells_total * sizeof(st::CellSlot)), "cell arena");
-  ST_CUDA(ensure(c->z_bins, (size_t)bins_total * 4), "z bins");
-  ST_CUDA(ensure(c->z_wins, (size_t)wins_total * 8), "window lists");
+  ST_CUDA(ensure(c->z_lists, (size_t)wins_total * 8 + (size_t)bins_total * 4), "window lists");
+  c->z_bins = (uint32_t*)((char*)c->z_lists.p + (size_t)wins_total * 8);
   ST_CUDA(ensure(c->d_blk_off, (size_t)blk[nj] * 8), "prepare block offsets");
   ST_CUDA(ensure(c->d_counter, 16), "work counter");
   ST_CUDA(ensure(c->d_err, 16), "error flags");
@@ -530,15 +530,15 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   pp.blk_count = (int32_t*)c->d_blk_count.p;
   pp.blk_offset = (int64_t*)c->d_blk_off.p;
   pp.cells = (st::CellSlot*)c->c_cells.p;
-  pp.bins = (uint32_t*)c->z_bins.p;
-  pp.wins = (unsigned long long*)c->z_wins.p;
+  pp.bins = c->z_bins;
+  pp.wins = (unsigned long long*)c->z_lists.p;
   pp.win_tiles = win_tiles;
   pp.any_flags = (int32_t*)((char*)c->d_counter.p + 8);
-  pp.PG = (int2*)c->pg.p;
-  pp.PGZ = (float*)c->pgz.p;
-  pp.PSRC = (uint32_t*)c->psrc.p;
-  pp.PV = (ulonglong2*)c->pv.p;
-  pp.PKEY = (unsigned long long*)c->pkey.p;
+  pp.PV = (ulonglong2*)c->prep.p;
+  pp.PG = (int2*)(pp.PV + prep_total);
+  pp.PKEY = (unsigned long long*)(pp.PG + prep_total);
+  pp.PGZ = (float*)(pp.PKEY + prep_total);
+  pp.PSRC = (uint32_t*)(pp.PGZ + prep_total);
   pp.fp32 = c->precision == 32 ? 1 : 0;
   pp.flag_min_kept = c->flag_min_kept;
   pp.sort = c->sort_deposits;
@@ -625,7 +625,7 @@ st::ResetParams reset_params(st_ctx* c, size_t nj, bool want_export) {
   r.u_done = (unsigned int*)c->u_done.p;
   r.u_table = (unsigned int*)c->u_table.p;
   r.n_units = c->cache_units;
-  r.bins = (uint32_t*)c->z_bins.p;
+  r.bins = c->z_bins;
   r.n_bins = c->cache_bins;
   r.err = (unsigned int*)c->d_err.p;
   r.ex_count = want_export ? (unsigned int*)c->ex_count.p : nullptr;
@@ -1075,10 +1075,10 @@ st_status st_ctx_destroy(st_ctx* c) {
   if (!c) return ST_ERR_INVALID_ARGUMENT;
   cudaSetDevice(c->device);
   cudaStreamSynchronize(c->stream);
-  DevBuf* bufs[] = {&c->track_arena, &c->pg, &c->pgz, &c->psrc, &c->pv, &c->pkey,
+  DevBuf* bufs[] = {&c->track_arena, &c->prep,
                     &c->d_jobs, &c->d_aux, &c->d_hists, &c->d_items, &c->d_blk,
                     &c->d_counter, &c->d_err, &c->d_blk_count, &c->d_blk_off, &c->d_blk_job, &c->c_cells,
-                    &c->z_bins, &c->z_wins, &c->u_next, &c->u_done, &c->u_table,
+                    &c->z_lists, &c->u_next, &c->u_done, &c->u_table,
                     &c->pool, &c->d_plan, &c->d_plan_misc, &c->g_keys, &c->g_lo, &c->g_hi,
                     &c->g_used, &c->g_count, &c->ex_buf, &c->ex_count, &c->h_counts,
                     &c->h_yfy, &c->h_edges};
