@@ -293,6 +293,14 @@ st_status upload_host_tracks(st_ctx* c, size_t first, size_t last, int64_t arena
   return ST_OK;
 }
 
+// Deposit*oversamples of jobs [first, last) per CTA.
+int64_t cta_share(const st_ctx* c, size_t first, size_t last, int grid) {
+  double units = 0;
+  for (size_t j = first; j < last; ++j)
+    units += (double)c->jobs[j].track.n * (double)c->jobs[j].desc.n_oversamples;
+  return (int64_t)std::min(units / grid, 9e17);
+}
+
 // Builds the device tables (jobs, aux, histograms, work items, prepare blocks) of jobs
 // [first, last) and the launch parameters; stores them in the context cache.
 st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
@@ -533,6 +541,10 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   pp.bins = c->z_bins;
   pp.wins = (unsigned long long*)c->z_lists.p;
   pp.win_tiles = win_tiles;
+  // (with share_divisor 0 no oversample is ever spread over CTAs)
+  pp.unit_min = c->share_divisor > 0
+                    ? c->min_chunks * st::chunk_tiles(c->chunk_windows) * st::kWarpTile : INT64_MAX;
+  pp.cta_share = cta_share(c, first, last, std::max(1, grid));
   pp.any_flags = (int32_t*)((char*)c->d_counter.p + 8);
   pp.PV = (ulonglong2*)c->prep.p;
   pp.PG = (int2*)(pp.PV + prep_total);
@@ -685,6 +697,7 @@ st_status enqueue_groups(st_ctx* c, const st::FusedParams& fp, size_t first,
     pp.blk_prefix += j0;
     pp.job_base = (int32_t)j0;
     pp.blk_base = c->cache_blk[j0];
+    pp.cta_share = cta_share(c, groups[g], groups[g + 1], std::max(1, c->cache_grid));
     bool flagged = false;
     for (size_t j = j0; j < j1; ++j) flagged |= c->cache_flagged[j] != 0;
     ST_CUDA(st::launch_prepare(pp, c->cache_blk[j1] - c->cache_blk[j0], flagged, false, c->stream), "prepare launch");

@@ -25,6 +25,21 @@ __device__ __forceinline__ bool coarse_windows(const JobDev& J, const JobAux& A)
   return A.windowed == kWinFlags && (J.cell_nbr8 ? 4 : 2) * (long long)A.cells < A.kept;
 }
 
+// A bin belongs to one CTA per oversample, so in a launch with too few oversamples to go round, a
+// layered job takes as long as its largest bin, while boundary flags spread an oversample over the
+// CTAs by chunks. Measured there (one track, 148 CTAs): layers 0.1 ms + 0.95 ns per deposit of the
+// largest bin, flags 0.6 ns per kept deposit. Dense tracks across z, layers / flags, fused: 1e6
+// deposits, 30 nm, 4 oversamples (nearly all in one bin) 0.80 / 0.48 ms; 300,007, 30 nm, 10 (two
+// bins) 0.27 / 0.15; 600,000, 20 nm, 10 (two) 0.31 / 0.34; 2e6, 20 nm, 4 (two) 0.90 / 1.25; 4e6,
+// 10 nm, 4 (two) 1.99 / 2.56. With CTAs enough at work, layers take three quarters of flags' time.
+// (Chunks of a layered bin that meet in a spill table took 4.2 ms on the last one.)
+__device__ __forceinline__ bool one_bin_too_large(const PrepareParams& p, long long kept,
+                                                  long long largest) {
+  const long long fixed = 84 << 10;
+  return kept > p.unit_min && 3 * largest > kept && 100 * (largest + fixed) > 63 * kept &&
+         10 * (largest + fixed) > 13 * p.cta_share;
+}
+
 // One CTA per job: exclusive scan of the job's block counts.
 __global__ void __launch_bounds__(1024) k_prep_scan(PrepareParams p) {
   chain_start();
@@ -70,13 +85,14 @@ __global__ void __launch_bounds__(1024) k_prep_scan(PrepareParams p) {
     uint32_t* bins = p.bins + p.jobs[j].bin_off;
     const int nb = p.jobs[j].n_bins;
     constexpr int kPer = kMaxBins / 1024;
-    unsigned v[kPer], sum = 0, big = 0;
+    unsigned v[kPer], sum = 0, big = 0, most = 0;
 #pragma unroll
     for (int t = 0; t < kPer; ++t) {
       const int b = (int)threadIdx.x * kPer + t;
       v[t] = b < nb ? bins[b] : 0;
       sum += v[t];
       big += v[t] > (unsigned)(2 * kWindow) ? v[t] : 0;
+      most = max(most, v[t]);
     }
     unsigned incl = sum;
 #pragma unroll
@@ -86,10 +102,15 @@ __global__ void __launch_bounds__(1024) k_prep_scan(PrepareParams p) {
     }
     __shared__ unsigned s_bin[32];
     __shared__ unsigned long long s_big;
-    if (threadIdx.x == 0) s_big = 0;
+    __shared__ unsigned s_most;
+    if (threadIdx.x == 0) {
+      s_big = 0;
+      s_most = 0;
+    }
     if (lane == 31) s_bin[warp] = incl;
     __syncthreads();
     if (big) atomicAdd(&s_big, (unsigned long long)big);
+    if (most) atomicMax(&s_most, most);
     unsigned base = incl - sum;
     for (int w = 0; w < warp; ++w) base += s_bin[w];
 #pragma unroll
@@ -108,7 +129,8 @@ __global__ void __launch_bounds__(1024) k_prep_scan(PrepareParams p) {
     // per diameter) 5.5 / 5.4, 4e6, 10 nm (4,000) 9.4 / 13.5, 2e6, 20 nm (8,000) 3.5 / 7.6.
     const JobDev& J = p.jobs[j];
     const bool dense = (double)J.n * J.d > 1024.0 * 2.0 * J.HL;
-    if (mode == kWinNone || dense || 4 * s_big <= (unsigned long long)kept) mode = kWinLayers;
+    const bool layers = dense || 4 * s_big <= (unsigned long long)kept;
+    if (mode == kWinNone || (layers && !one_bin_too_large(p, kept, s_most))) mode = kWinLayers;
   }
   if (threadIdx.x == 0) {
     p.aux[j].kept = kept;
@@ -184,14 +206,6 @@ __device__ __forceinline__ void cut_windows(const PrepareParams& p, const JobDev
 // threads could part ways there.
 __device__ __forceinline__ bool cta_over(const int* count, int limit) {
   return __syncthreads_or(*(const volatile int*)count > limit) != 0;
-}
-
-// Warp tiles of a shared unit's chunk: chunk_windows windows of kWinTiles tiles per warp,
-// rounded up to whole coarse windows, so that no window is ever split between two chunks.
-__host__ __device__ __forceinline__ int64_t chunk_tiles(int chunk_windows) {
-  constexpr int64_t kCoarse = (int64_t)kFusedWarps * kCoarseTiles;
-  const int64_t t = (int64_t)chunk_windows * kFusedWarps * kWinTiles;
-  return (t + kCoarse - 1) / kCoarse * kCoarse;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -283,6 +283,9 @@ struct PrepareParams {
   uint32_t* bins;             // z bins of layered jobs: kept deposits, then first free place
   unsigned long long* wins;   // window lists of layered jobs
   int32_t win_tiles;          // warp tiles of a layer window (twice that on dense tracks)
+  int64_t cta_share;          // deposit*oversamples of the launch per CTA of the fused kernel
+  int64_t unit_min;           // kept deposits above which an oversample of a job with boundary flags
+                              // is spread over CTAs (a shared unit)
   int32_t* any_flags;         // set when a job of the launch runs with window boundary flags
   int2* PG;                   // records as in FusedParams
   float* PGZ;
@@ -361,6 +364,14 @@ constexpr int kCtaTile = kFusedWarps * kWarpTile;    // kept deposits of one war
 constexpr int kWinTiles = 2;                          // warp tiles per warp in a window
 constexpr int kCoarseTiles = 4;                       // ... in a coarse window (dense spheres)
 constexpr int kWindow = kWinTiles * kCtaTile;         // kept deposits per window (8192)
+// Warp tiles of a shared unit's chunk: chunk_windows windows of kWinTiles tiles per warp,
+// rounded up to whole coarse windows, so that no window is ever split between two chunks.
+ST_HD int64_t chunk_tiles(int chunk_windows) {
+  constexpr int64_t kCoarse = (int64_t)kFusedWarps * kCoarseTiles;
+  const int64_t t = (int64_t)chunk_windows * kFusedWarps * kWinTiles;
+  return (t + kCoarse - 1) / kCoarse * kCoarse;
+}
+
 // A flagged job uses flag cells of side 2d (eight probes per deposit instead of 27, but more
 // deposits flagged, whose spheres then pass through the spill log at every oversample) when its
 // deposits per sphere diameter of track length, n * d / (2 HL), times its oversamples are at most

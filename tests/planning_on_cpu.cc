@@ -63,6 +63,46 @@ int plan_batch(int n_jobs, const int64_t* kept, const int32_t* n_os, const int32
   return n_items;
 }
 
+// Window mode that k_prep_scan gives a job with these z bins (the kept deposits of all); the bins
+// become their first places.
+int window_mode(int n_bins, uint32_t* bins, double per_diameter, int64_t cta_share, int64_t unit_min,
+                const int32_t* order) {
+  st::JobDev job;
+  st::JobAux aux;
+  st::PrepareParams p;
+  std::memset(&job, 0, sizeof(job));
+  std::memset(&aux, 0, sizeof(aux));
+  std::memset(&p, 0, sizeof(p));
+  int64_t kept = 0;
+  for (int b = 0; b < n_bins; ++b) kept += bins[b];
+  const int blocks = (int)((kept + 1023) / 1024);
+  std::vector<int32_t> count(blocks, 1024);
+  if (blocks) count.back() = (int32_t)(kept - (blocks - 1) * 1024ll);
+  std::vector<int64_t> offset(blocks);
+  const int64_t prefix[2] = {0, blocks};
+  int32_t any = 0;
+  job.n = kept;
+  job.d = per_diameter / kept;  // n * d / (2 HL) deposits per sphere diameter
+  job.HL = 0.5;
+  job.flagged = job.layers = 1;
+  job.n_bins = n_bins;
+  p.jobs = &job;
+  p.aux = &aux;
+  p.n_jobs = 1;
+  p.blk_prefix = prefix;
+  p.blk_count = count.data();
+  p.blk_offset = offset.data();
+  p.bins = bins;
+  p.any_flags = &any;
+  p.flag_min_kept = 16384;
+  p.cta_share = cta_share;
+  p.unit_min = unit_min;
+  emu::run_cta(1024, dim3(1), 0, warps(32, order), [&] { st::k_prep_scan(p); });
+  for (int b = 0; b < blocks; ++b)
+    if (offset[b] != b * 1024ll) return -1;
+  return aux.kept == kept && any == (aux.windowed == st::kWinFlags) ? aux.windowed : -2;
+}
+
 // Windows of a CTA that adds `per_window` to a count in each and empties it above `limit` (cta_over).
 // Returns how many threads took another branch than thread 0 at some window's end.
 int empty_windows(int windows, int per_window, int limit, const int32_t* order) {

@@ -95,6 +95,36 @@ def test_plan_covers_every_window_once(lib, kept, n_os, n_win, grid):
     assert np.all(done == 1)
 
 
+NONE, FLAGS, LAYERS = range(3)
+# z bins, deposits per sphere diameter, deposit*oversamples per CTA, mode
+TRACKS = {
+    "along z": ([300] * 1000, 3000.0, 20_000, LAYERS),
+    "few deposits": ([16_384], 3000.0, 20_000, NONE),
+    "dense, in one bin, 4 oversamples": ([900_000] + [1000] * 100, 3000.0, 27_000, FLAGS),
+    "the same with shared units off": ([900_000] + [1000] * 100, 3000.0, 27_000, LAYERS),
+    "the same, 148 oversamples": ([900_000] + [1000] * 100, 3000.0, 1_000_000, LAYERS),
+    "dense, in two bins, 10 oversamples": ([135_000] * 2 + [300] * 100, 1800.0, 20_000, FLAGS),
+    "dense, in two bins, large": ([900_000] * 2 + [2000] * 100, 4000.0, 54_000, LAYERS),
+    "dense, in eight bins": ([40_000] * 8, 1800.0, 8_000, LAYERS),
+    "dense, in one bin, too small for units": ([120_000], 1800.0, 3_000, LAYERS),
+    "sparse, a third in large bins": ([400] * 300 + [20_000] * 3, 500.0, 5_000, FLAGS),
+    "sparse, a fifth in large bins": ([400] * 300 + [30_000], 500.0, 5_000, LAYERS),
+}
+
+
+@pytest.mark.parametrize("order", sorted(ORDERS))
+@pytest.mark.parametrize("track", sorted(TRACKS))
+def test_window_mode(lib, track, order):
+    """Layers, unless they would leave most CTAs without work or empty bins into the log."""
+    sizes, per_d, share, mode = TRACKS[track]
+    bins = np.array(sizes, dtype=np.uint32)
+    unit_min = (1 << 62) if "units off" in track else 4 * 32_768
+    assert lib.window_mode(len(bins), _ptr(bins), C.c_double(per_d), C.c_int64(share),
+                           C.c_int64(unit_min), _ptr(_order(order))) == mode
+    if sum(sizes) > 16_384:
+        assert np.array_equal(bins, np.concatenate([[0], np.cumsum(sizes)[:-1]]))
+
+
 def test_footprint_charges_what_a_job_allocates(lib):
     """st_server_job_footprint against the arrays of a context that grow with a job; and no more
     than 48 bytes of records per deposit and 8 of a qualifying job's shifted z came to, so that what
