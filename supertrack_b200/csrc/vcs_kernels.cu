@@ -234,6 +234,26 @@ __device__ __forceinline__ bool cells_foreign(const PrepareParams& p, const JobD
   return foreign;
 }
 
+// The z bins that a prepare block meets, in shared memory: the block adds to a bin's word in HBM once
+// instead of once per warp or cell group, which on tracks across z all meet on a few words (prepare
+// of one track of 4e6 deposits, 10 nm, across z 0.69 -> 0.27 ms, along z 0.39 -> 0.23). A bin that finds its
+// place taken four times goes to HBM directly; a block of many bins is no contention.
+constexpr int kBlockBins = 64;
+__device__ __forceinline__ int block_bin(int* keys, int bin) {
+  int h = bin & (kBlockBins - 1);
+#pragma unroll 1
+  for (int probe = 0; probe < 4; ++probe) {
+    int k = *(volatile int*)&keys[h];
+    if (k < 0) {
+      k = atomicCAS(&keys[h], -1, bin);
+      if (k < 0) k = bin;
+    }
+    if (k == bin) return h;
+    h = (h + 1) & (kBlockBins - 1);
+  }
+  return -1;
+}
+
 // Eight blocks per SM (32 registers): more track loads in flight.
 __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_count(PrepareParams p) {
   chain_start();
@@ -242,6 +262,15 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_count(PrepareParams p)
   const JobDev J = p.jobs[j];
   const int64_t i0 = (b - p.blk_prefix[j]) * (int64_t)kPrepSlotsPerBlock;
   int emin = INT_MAX, emax = INT_MIN, flags = 0, kept = 0;
+  __shared__ int s_key[kBlockBins];
+  __shared__ unsigned s_count[kBlockBins];
+  if (J.layers) {
+    if (threadIdx.x < kBlockBins) {
+      s_key[threadIdx.x] = -1;
+      s_count[threadIdx.x] = 0;
+    }
+    __syncthreads();
+  }
   // a guard rather than a break, so that the loads of all rounds can be in flight together
 #pragma unroll
   for (int s = threadIdx.x; s < kPrepSlotsPerBlock; s += kPrepThreads) {
@@ -255,8 +284,10 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_count(PrepareParams p)
       // met on the same words: 7.9 ms instead of about 1.6 for 32e6 deposits of 10 nm ion tracks)
       const int bin = keep ? z_bin(J, st_dadd(z, J.zsh)) : -1;
       const unsigned same = __match_any_sync(0xffffffffu, bin);
-      if (keep && (int)(threadIdx.x & 31) == __ffs(same) - 1)
-        atomicAdd(&p.bins[J.bin_off + bin], (unsigned)__popc(same));
+      if (keep && (int)(threadIdx.x & 31) == __ffs(same) - 1) {
+        const int q = block_bin(s_key, bin);
+        atomicAdd(q >= 0 ? &s_count[q] : &p.bins[J.bin_off + bin], (unsigned)__popc(same));
+      }
     }
     if (!in) continue;
     const double v = __ddiv_rn(J.edep[i], J.denom);
@@ -295,6 +326,8 @@ __global__ void __launch_bounds__(kPrepThreads, 8) k_prep_count(PrepareParams p)
     }
   }
   __syncthreads();
+  if (J.layers && threadIdx.x < kBlockBins && s_count[threadIdx.x])
+    atomicAdd(&p.bins[J.bin_off + s_key[threadIdx.x]], s_count[threadIdx.x]);
   if (threadIdx.x == 0) {
     p.blk_count[b] = s_kept;
     if (s_flags) {
@@ -381,7 +414,10 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
   __shared__ unsigned s_first[kCellHashBins];
   __shared__ unsigned s_group[kPrepSlotsPerBlock];
   __shared__ unsigned s_part[kWarpsPerBlock];
-  __shared__ unsigned s_base[kPrepSlotsPerBlock];  // layered jobs: first place of each group
+  // layered jobs: first place of each group, or with bit 31 its block bin and offset there
+  __shared__ unsigned s_base[kPrepSlotsPerBlock];
+  __shared__ int s_key[kBlockBins];          // block bins, the deposits of each and its first place
+  __shared__ unsigned s_count[kBlockBins], s_place[kBlockBins];
   __shared__ unsigned short s_zbin[kPrepSlotsPerBlock];  // and its z bin
   int64_t run = p.blk_offset[b];  // kept index of the next kept deposit of this block
   const JobAux A = p.aux[j];
@@ -392,6 +428,10 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
     for (int t = 0; t < kHashPerThread; ++t) s_first[threadIdx.x * kHashPerThread + t] = ~0u;
 #pragma unroll
     for (int t = 0; t < kGroupsPerThread; ++t) s_group[threadIdx.x * kGroupsPerThread + t] = 0;
+    if (threadIdx.x < kBlockBins) {
+      s_key[threadIdx.x] = -1;
+      s_count[threadIdx.x] = 0;
+    }
   }
   const int E0 = choose_grid_exponent(A.e_min, A.e_max, J.n, A.flags & kAuxNonzero);
   unsigned created_cells = 0;  // cells this thread created (windowed jobs)
@@ -450,10 +490,15 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
     for (int r = 0; r < kRounds; ++r) {
       const unsigned own = r * kPrepThreads + threadIdx.x;
       if ((keep & (1u << r)) && (slot_of[r] >> 16) == own) {
-        s_base[own] = atomicAdd(&p.bins[J.bin_off + s_zbin[own]], s_group[own]);
+        const int bin = s_zbin[own], q = block_bin(s_key, bin);
+        s_base[own] = q >= 0 ? 0x80000000u | q << 16 | atomicAdd(&s_count[q], s_group[own])
+                             : atomicAdd(&p.bins[J.bin_off + bin], s_group[own]);
         ++created_cells;
       }
     }
+    __syncthreads();
+    if (threadIdx.x < kBlockBins && s_count[threadIdx.x])
+      s_place[threadIdx.x] = atomicAdd(&p.bins[J.bin_off + s_key[threadIdx.x]], s_count[threadIdx.x]);
     __syncthreads();
   } else if (sorted) {
 #pragma unroll
@@ -503,7 +548,9 @@ __global__ void __launch_bounds__(kPrepThreads, 4) k_prep_write(PrepareParams p)
     if (keep & (1u << r)) {
       // kept index: block order, or the position of the deposit's group and rank in sorted
       // blocks
-      const int64_t k = layered ? (int64_t)s_base[slot_of[r] >> 16] + (slot_of[r] & 0xFFFFu)
+      const unsigned first = layered ? s_base[slot_of[r] >> 16] : 0;
+      const int64_t k = layered ? (int64_t)(first >> 31 ? s_place[first >> 16 & (kBlockBins - 1)] + (first & 0xFFFFu)
+                                                        : first) + (slot_of[r] & 0xFFFFu)
                         : sorted ? p.blk_offset[b] + s_group[slot_of[r] >> 16] + (slot_of[r] & 0xFFFFu)
                                : run + before + __popc(m[r] & ((1u << lane) - 1u));
       const double az = st_dsub(z1[r], J.gSO);
