@@ -17,6 +17,7 @@
 namespace st {
 cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_flagged,
                            bool chained, cudaStream_t s);
+int prepare_launches(int64_t n_blocks, bool any_flagged);
 cudaError_t configure_fused();
 bool fused_big_table(int max_nbins, int table_slots);
 cudaError_t launch_fused(FusedParams p, int max_nbins, int grid, int table_slots, cudaStream_t s);
@@ -203,7 +204,6 @@ struct st_ctx {
   int cache_max_nbins = 0;
   int64_t cache_cells = 0;
   int64_t cache_bins = 0;
-  bool cache_any_flagged = false;
   int64_t cache_units = 0;
   int64_t cache_item_cap = 0;
   st::PlanParams cache_plan{};
@@ -333,7 +333,6 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   std::vector<JobDev> jd(nj);
   std::vector<int64_t> blk(nj + 1, 0);
   int64_t cells_total = 0, bins_total = 0, wins_total = 0;
-  bool any_flagged = false;
   // layer windows of two warp tiles per warp, one on the table of half the slots
   int max_nbins = 0;
   for (size_t i = 0; i < nj; ++i)
@@ -402,7 +401,6 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
       D.cell_cap = next_pow2((uint64_t)2 * (uint64_t)J.track.n);
       D.cell_off = cells_total;
       cells_total += D.cell_cap;
-      any_flagged = true;
     }
     D.bin_off = bins_total;
     D.win_off = wins_total;
@@ -594,7 +592,6 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   c->cache_arena_total = arena_total;
   c->cache_cells = cells_total;
   c->cache_bins = bins_total;
-  c->cache_any_flagged = any_flagged;
   c->cache_units = units;
   // planner parameters; the scratch block holds total_units (8 B), n_items (4 B), the unit
   // counter (4 B) and the three bucket arrays
@@ -644,6 +641,11 @@ st::ResetParams reset_params(st_ctx* c, size_t nj, bool want_export) {
   return r;
 }
 
+// Whether any of jobs [j0, j1) of the launch, counted from its first, may run with boundary flags.
+bool any_flagged(const st_ctx* c, size_t j0, size_t j1) {
+  return std::any_of(c->cache_flagged.begin() + j0, c->cache_flagged.begin() + j1, [](char f) { return f != 0; });
+}
+
 // Enqueues the device side of a run on the context's stream: the resets, the prepare, plan and
 // fused kernels, and the copies of the job counters and error flags into pinned host memory,
 // with the run's events. Nothing waits; finish_range picks the results up. While the stream is
@@ -654,7 +656,7 @@ st_status enqueue_run(st_ctx* c, const st::FusedParams& fp, size_t nj, bool want
   ST_CUDA(st::launch_reset(reset_params(c, nj, want_export), c->stream), "reset");
 
   ST_CUDA(cudaEventRecordWithFlags(c->ev[0], c->stream, evf), "event");
-  ST_CUDA(st::launch_prepare(c->cache_pp, c->cache_blocks, c->cache_any_flagged, false, c->stream), "prepare launch");
+  ST_CUDA(st::launch_prepare(c->cache_pp, c->cache_blocks, any_flagged(c, 0, nj), false, c->stream), "prepare launch");
   ST_CUDA(st::launch_plan(c->cache_plan, c->cache_blocks > 0, c->stream), "plan launch");
   ST_CUDA(cudaEventRecordWithFlags(c->ev[1], c->stream, evf), "event");
   if (c->order_after && !capturing) {
@@ -698,9 +700,7 @@ st_status enqueue_groups(st_ctx* c, const st::FusedParams& fp, size_t first,
     pp.job_base = (int32_t)j0;
     pp.blk_base = c->cache_blk[j0];
     pp.cta_share = cta_share(c, groups[g], groups[g + 1], std::max(1, c->cache_grid));
-    bool flagged = false;
-    for (size_t j = j0; j < j1; ++j) flagged |= c->cache_flagged[j] != 0;
-    ST_CUDA(st::launch_prepare(pp, c->cache_blk[j1] - c->cache_blk[j0], flagged, false, c->stream), "prepare launch");
+    ST_CUDA(st::launch_prepare(pp, c->cache_blk[j1] - c->cache_blk[j0], any_flagged(c, j0, j1), false, c->stream), "prepare launch");
     st::PlanParams q = c->cache_plan;
     q.jobs += j0;
     q.aux += j0;
@@ -878,9 +878,11 @@ st_status launch_range(st_ctx* c, size_t first, size_t last, bool want_export, i
     if (s != ST_OK) return s;
   }
   const size_t n_groups = groups.size() - 1;
-  for (size_t g = 0; g < n_groups; ++g)
-    c->launches += 1 + (c->cache_blocks > 0 ? (c->cache_any_flagged ? 6 : 4) : 0) +
-                   st::plan_launches((int)(groups[g + 1] - groups[g])) + (c->cache_grid > 0 ? 1 : 0);
+  for (size_t g = 0; g < n_groups; ++g) {
+    const size_t j0 = groups[g] - first, j1 = groups[g + 1] - first;
+    c->launches += 1 + st::prepare_launches(c->cache_blk[j1] - c->cache_blk[j0], any_flagged(c, j0, j1)) +
+                   st::plan_launches((int)(j1 - j0)) + (c->cache_grid > 0 ? 1 : 0);
+  }
   c->pending = true;
   c->pend_first = first;
   c->pend_last = last;

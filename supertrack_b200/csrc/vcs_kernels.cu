@@ -1906,6 +1906,10 @@ size_t fused_smem_bytes(int cap, int hist_bins) {
   return (size_t)cap * 26 + (size_t)cap / 8 + (size_t)hist_bins * 28 + 8;
 }
 
+int prepare_launches(int64_t n_blocks, bool any_flagged) {
+  return n_blocks <= 0 ? 0 : any_flagged ? 6 : 4;
+}
+
 cudaError_t launch_prepare(const PrepareParams& p, int64_t n_blocks, bool any_flagged,
                            bool chained, cudaStream_t s) {
   if (n_blocks <= 0) return cudaSuccess;
