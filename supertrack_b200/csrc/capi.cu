@@ -202,7 +202,6 @@ struct st_ctx {
   int cache_grid = 0;
   int64_t cache_arena_total = 0;
   int cache_max_nbins = 0;
-  int64_t cache_cells = 0;
   int64_t cache_bins = 0;
   int64_t cache_units = 0;
   int64_t cache_item_cap = 0;
@@ -452,7 +451,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   ST_CUDA(ensure(c->u_table, (size_t)units * 4), "units");
   ST_CUDA(ensure(c->d_items, (size_t)item_cap * sizeof(WorkItem)), "items");
   ST_CUDA(ensure(c->d_plan, nj * sizeof(st::JobPlan)), "plan");
-  ST_CUDA(ensure(c->d_plan_misc, 4096), "plan scratch");
+  ST_CUDA(ensure(c->d_plan_misc, st::kPlanScratch), "plan scratch");
 
   ST_CUDA(ensure(c->d_jobs, nj * sizeof(JobDev)), "job table");
   ST_CUDA(ensure(c->d_aux, nj * sizeof(JobAux)), "job aux");
@@ -558,7 +557,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   fp.aux = pp.aux;
   fp.hists = (const HistDev*)c->d_hists.p;
   fp.items = (const WorkItem*)c->d_items.p;
-  fp.n_items = (const int*)((char*)c->d_plan_misc.p + 8);
+  fp.n_items = (const int*)c->d_plan_misc.p;
   fp.flush_threshold = 1024;
   fp.work_counter = (unsigned int*)c->d_counter.p;
   fp.PG = pp.PG; fp.PGZ = pp.PGZ;
@@ -590,11 +589,9 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   c->cache_grid = work_jobs == 0 ? 0 : grid;
   c->cache_item_cap = item_cap;
   c->cache_arena_total = arena_total;
-  c->cache_cells = cells_total;
   c->cache_bins = bins_total;
   c->cache_units = units;
-  // planner parameters; the scratch block holds total_units (8 B), n_items (4 B), the unit
-  // counter (4 B) and the three bucket arrays
+  // planner parameters (scratch block: see kPlanScratch)
   st::PlanParams& q = c->cache_plan;
   char* m = (char*)c->d_plan_misc.p;
   q.jobs = (const JobDev*)c->d_jobs.p;
@@ -606,11 +603,9 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
   q.item_cost = c->item_cost;
   q.share_divisor = c->share_divisor;
   q.min_chunks = c->min_chunks;
-  q.total_units = (unsigned long long*)m;
-  q.n_items = (int*)(m + 8);
-  q.unit_counter = (unsigned int*)(m + 12);
-  q.bucket_count = (unsigned int*)(m + 16);
-  q.bucket_start = q.bucket_count + st::kPlanBuckets;
+  q.n_items = (int*)m;
+  q.unit_counter = (unsigned int*)(m + 4);
+  q.bucket_start = (unsigned int*)(m + 8);
   q.bucket_cursor = q.bucket_start + st::kPlanBuckets;
   q.plan = (st::JobPlan*)c->d_plan.p;
   q.items = (WorkItem*)c->d_items.p;

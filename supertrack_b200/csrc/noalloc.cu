@@ -93,7 +93,7 @@ constexpr Layout make_layout() {
   L.pool = o;       o += al(4);
   L.items = o;      o += al((size_t)kNaMaxOversamples * sizeof(st::WorkItem));
   L.plan = o;       o += al(sizeof(st::JobPlan));
-  L.plan_misc = o;  o += al(16 + 3 * 4 * st::kPlanBuckets);
+  L.plan_misc = o;  o += al(st::kPlanScratch);
   L.counter = o;    o += al(16);
   L.units = o;      o += al(3 * 4);
   L.total = o;
@@ -301,11 +301,9 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   // deliberate difference from the regular path: share_divisor 0 (left zero) rules out shared
   // units, whose helpers would need a spill table each from a pool of one table per CTA;
   // min_chunks only matters for shared units
-  q.total_units = (unsigned long long*)m;
-  q.n_items = (int*)(m + 8);
-  q.unit_counter = (unsigned int*)(m + 12);
-  q.bucket_count = (unsigned int*)(m + 16);
-  q.bucket_start = q.bucket_count + st::kPlanBuckets;
+  q.n_items = (int*)m;
+  q.unit_counter = (unsigned int*)(m + 4);
+  q.bucket_start = (unsigned int*)(m + 8);
   q.bucket_cursor = q.bucket_start + st::kPlanBuckets;
   q.plan = (st::JobPlan*)(base + L.plan);
   q.items = (st::WorkItem*)(base + L.items);

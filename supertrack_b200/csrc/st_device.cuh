@@ -320,8 +320,6 @@ struct PlanParams {
   long long item_cost;
   int32_t share_divisor;             // a job is shared when kept > total / (share_divisor * grid)
   int32_t min_chunks;                // ... and kept > min_chunks chunks; share_divisor 0: never
-  unsigned long long* total_units;   // sum of kept * n_os
-  unsigned int* bucket_count;        // kPlanBuckets
   unsigned int* bucket_start;        // kPlanBuckets
   unsigned int* bucket_cursor;       // kPlanBuckets
   unsigned int* unit_counter;
@@ -355,7 +353,8 @@ struct ResetParams {
   int64_t n_slots;
   int32_t n_tables;
 };
-constexpr int kPlanScratch = 16 + 3 * 4 * kPlanBuckets;  // bytes
+// the planner's scratch: item count, unit counter, buckets' starts and cursors, in bytes
+constexpr int kPlanScratch = 8 + 2 * 4 * kPlanBuckets;
 
 constexpr int kPrepThreads = 256;
 constexpr int kPrepSlotsPerBlock = 1024;                // source deposits per prepare block

@@ -1,10 +1,10 @@
 // sm_100a kernels of the VoxelConstrainedSphere superimposition path.
 //
-//   prepare   : once per track (k_prep_count/scan/write/pad). z-origin shift, the deposits that
-//               can be in the voxel for some shift, the z part of the lattice test (k_z and
-//               (k_z*d - a_z)^2, which do not depend on the oversample), the lineal energy
-//               contribution v = edep/((2/3)d), the job's fixed-point exponent range, and the
-//               ordered compaction of the kept deposits into the prepared arena.
+//   prepare   : once per run of a track (k_prep_*). z-origin shift, the deposits that
+//               can be in the voxel for some shift, x and y in lattice units, the z part of the
+//               lattice test (k_z and (k_z*d - a_z)^2, which do not depend on the oversample), the
+//               lineal energy contribution v = edep/((2/3)d), the job's fixed-point exponent range,
+//               and the compaction of the kept deposits into the prepared arena.
 //               Follows VoxelConstrainedSphereMethod.cu:138-154 (z shift), :198 (|z| test),
 //               :249-258 (z axis of the membership test), :302/:322 (lineal denominator).
 //   k_fused   : persistent work-stealing kernel over (job, oversample block) items. Per
@@ -51,15 +51,21 @@ __device__ __forceinline__ double lattice_index(double a, double d, double inv_d
 }
 
 // ---------------------------------------------------------------------------------------------
-// Prepare stage (once per track): four launches.
+// Prepare stage (once per run of a track): four launches, six when a job may run with boundary flags.
 //   k_prep_count : per block of kPrepSlotsPerBlock source deposits, the number of deposits that
 //                  can lie inside the voxel for some oversample (z after the z-origin shift
 //                  strictly inside; |x|, |y| below xy_keep), plus the job's exponent range of
-//                  the contributions v = edep/((2/3)d) over all its deposits;
-//   k_prep_scan  : per job, exclusive scan of its block counts -> block offsets, kept total;
-//   k_prep_write : ordered compaction of the kept deposits into the prepared arena with
-//                  the oversample-independent z part of the lattice test;
-//   k_prep_pad   : padding of each job's last warp tile (NaN x so the box test rejects it).
+//                  the contributions v = edep/((2/3)d) over all its deposits, and the z bins of
+//                  jobs that qualify for layer windows;
+//   k_prep_scan  : per job, exclusive scan of its block counts -> block offsets, kept total, window
+//                  mode (planning.cuh);
+//   k_prep_cells : empties the cell hashes of jobs with boundary flags;
+//   k_prep_write : compaction of the kept deposits into the prepared arena (source order, grouped
+//                  by cell, or by z layer) with the oversample-independent z part of the lattice
+//                  test, and the cells of jobs with boundary flags;
+//   k_prep_pad   : padding of each job's last warp tile (outside the voxel for every shift), and the
+//                  window lists of layered jobs;
+//   k_prep_flag  : the boundary flags.
 // A dropped deposit can be inside the box for no shift, so dropping it changes no result.
 // ---------------------------------------------------------------------------------------------
 __device__ __forceinline__ int find_job(const int64_t* blk_prefix, int n_jobs, int64_t b) {
