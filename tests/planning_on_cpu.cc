@@ -4,6 +4,7 @@
 // (after the emulator's intrinsics)
 #include "../supertrack_b200/csrc/planning.cuh"
 
+#include <cmath>
 #include <cstring>
 
 namespace {
@@ -101,6 +102,64 @@ int window_mode(int n_bins, uint32_t* bins, double per_diameter, int64_t cta_sha
   for (int b = 0; b < blocks; ++b)
     if (offset[b] != b * 1024ll) return -1;
   return aux.kept == kept && any == (aux.windowed == st::kWinFlags) ? aux.windowed : -2;
+}
+
+// The window list that cut_windows makes of a job's z bins (their ends) with `cells` occupied cells:
+// n_win + 1 entries. Returns n_win.
+int cut(int n_bins, const uint32_t* ends, int64_t cells, int win_tiles, uint64_t* wins) {
+  st::JobDev job;
+  st::JobAux aux;
+  st::PrepareParams p;
+  std::memset(&job, 0, sizeof(job));
+  std::memset(&aux, 0, sizeof(aux));
+  std::memset(&p, 0, sizeof(p));
+  job.n_bins = n_bins;
+  aux.kept = ends[n_bins - 1];
+  aux.cells = cells;
+  p.win_tiles = win_tiles;
+  static_assert(sizeof(unsigned long long) == sizeof(uint64_t), "");
+  p.wins = reinterpret_cast<unsigned long long*>(wins);
+  emu::run_cta(32, dim3(1), 0, {0}, [&] { st::cut_windows(p, job, &aux, ends); });
+  return aux.n_win;
+}
+
+// The integer geometry of deposits (x, y) and their z offsets dz in an oversample of shift (sx, sy),
+// with the constants of set_integer_geometry and the float steps of the fused kernel: bit 0 in the
+// voxel, bit 1 a hit, bit 2 left to FP64, and the sphere's indices. Returns g_shift.
+int integer_geometry(int n, int64_t lattice, double d, double gso, double sx, double sy, const double* x,
+                     const double* y, const double* dz, int32_t* decision, int32_t* kx, int32_t* ky) {
+  st::JobDev J;
+  std::memset(&J, 0, sizeof(J));
+  J.N = (uint32_t)lattice;
+  J.d = d;
+  st::set_integer_geometry(&J);
+  const int half = 1 << J.g_shift >> 1;
+  const int cx = (int)std::nearbyint((sx - gso) * J.g_scale) + half;
+  const int cy = (int)std::nearbyint((sy - gso) * J.g_scale) + half;
+  const unsigned in_max = (unsigned)J.g_ns - 4u, near_max = (unsigned)J.g_ns + 2u, low = (1u << J.g_shift) - 1u;
+  const float centre = 8388608.0f + (float)(1 << J.g_shift) * 0.5f;
+  const auto offset = [&](unsigned v) {
+    const unsigned bits = (v & low) | 0x4B000000u;
+    float f;
+    std::memcpy(&f, &bits, 4);
+    return f - centre;
+  };
+  for (int i = 0; i < n; ++i) {
+    const unsigned vx = (unsigned)(int)std::nearbyint(x[i] * J.g_scale) + (unsigned)cx;
+    const unsigned vy = (unsigned)(int)std::nearbyint(y[i] * J.g_scale) + (unsigned)cy;
+    const double gz = dz[i] * J.g_scale;
+    const float z2 = (float)(gz * gz);
+    const bool in = vx - 2u <= in_max && vy - 2u <= in_max;
+    const bool near = vx + 1u <= near_max && vy + 1u <= near_max;
+    const float fx = offset(vx), fy = offset(vy);
+    const float d2 = std::fma(fx, fx, std::fma(fy, fy, z2));
+    const bool hit = in && d2 <= J.g_lo;
+    const bool open = in ? (!hit && d2 <= J.g_hi) : near;
+    decision[i] = (in ? 1 : 0) | (hit ? 2 : 0) | (open ? 4 : 0);
+    kx[i] = (int)vx >> J.g_shift;
+    ky[i] = (int)vy >> J.g_shift;
+  }
+  return J.g_shift;
 }
 
 // Windows of a CTA that adds `per_window` to a count in each and empties it above `limit` (cta_over).

@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 from supertrack_b200 import _capi
+from test_integer_geometry_property import _deposits, _fp64, _geometry
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
@@ -197,3 +198,58 @@ def test_kept_sums_stay_below_128_bits(lib, ratio_bits, lower, work):
         assert total < 1 << 127
         back = _capi.lib().st_from_fixed(total & (2 ** 64 - 1), total >> 64, e0)
         assert back == float(y) * spheres
+
+
+@pytest.mark.parametrize("win_tiles", [32, 64])
+@pytest.mark.parametrize("m", [1, 3, 4, 5, 8, 100])
+def test_window_list(lib, m, win_tiles):
+    """cut_windows: windows that follow one another, end at the end of a bin or, inside one, at a
+    whole tile (the next one is then marked), span no more tiles than they may, and fit the arena."""
+    rng = np.random.default_rng(win_tiles * 100 + m)
+    tiles = (1 if m < 2 else 2 if m < 4 else min(m, 8)) * win_tiles
+    lists = [np.full(4096, s) for s in (1, 5, 127, 128, 129, 1000)]
+    for a in (1, 21, 22, 31, 32, 33, win_tiles):
+        for big in (12, 34, win_tiles + 1, 8 * win_tiles + 1):
+            lists.append(np.tile([a * 128, big * 128], 40))
+            lists.append(np.tile([a * 128 + 1, 0, big * 128 - 1, 3], 40))
+    for _ in range(20):
+        lists.append(rng.integers(0, 2 ** rng.integers(1, 18), size=rng.integers(1, 600)) + 1)
+        lists.append((rng.pareto(0.8, size=300) * 200).astype(np.int64) % 300_000 + 1)
+    lib.window_cap.restype = C.c_int64
+    for sizes in lists:
+        ends = np.cumsum(sizes).astype(np.uint32)
+        kept = int(ends[-1])
+        cap = lib.window_cap(C.c_int64(kept), C.c_int64(win_tiles * 128))
+        wins = np.zeros(2 * cap + 64, dtype=np.uint64)
+        n = lib.cut(len(ends), _ptr(ends), C.c_int64(max(kept // m, 1)), win_tiles, _ptr(wins))
+        assert n + 1 <= cap
+        first = (wins[:n + 1] & np.uint64(2 ** 63 - 1)).astype(np.int64)
+        inside = wins[:n + 1] >= np.uint64(2 ** 63)
+        assert first[0] == 0 and first[n] == kept and np.all(np.diff(first) > 0)
+        assert not inside[0] and not inside[n]
+        assert np.all(-(-first[1:] // 128) - first[:-1] // 128 <= tiles)
+        at_end = np.isin(first[1:], ends)
+        # (a cut inside a bin falls on a whole tile, which may happen to be a bin's end as well)
+        assert np.all(at_end | inside[1:]) and np.all(first[1:][inside[1:]] % 128 == 0)
+
+
+@pytest.mark.parametrize("hl,d", [(2500.0, 2.0), (2500.0, 1000.0), (5000.0, 10.0), (1.0, 2.0),
+                                  (3.0, 1000.0), (1e6, 1.0), (0.37, 1e-3), (5e12, 7e6)])
+def test_integer_geometry_with_the_kernel_constants(lib, hl, d):
+    """What set_integer_geometry lets the 32-bit integers and float sums decide, FP64 decides too."""
+    rs = np.random.default_rng(int(hl * 7 + d * 13) % 2 ** 32)
+    n, h, length, gso = _geometry(hl, d)
+    for u in (1.0, 2.0 ** -24, 0.5, *rs.random(3)):
+        sx, sy = u * length - h, rs.random() * length - h
+        x, y, dz = _deposits(rs, n, h, d, gso, sx, sy, 60_000)
+        out = [np.zeros(len(x), dtype=np.int32) for _ in range(3)]
+        f = C.c_double
+        lib.integer_geometry(len(x), C.c_int64(n), f(d), f(gso), f(sx), f(sy), _ptr(x), _ptr(y),
+                             _ptr(dz), *[_ptr(o) for o in out])
+        inb, hit, kx, ky = _fp64(x, y, dz, sx, sy, h, d, gso)
+        sure = out[0] & 4 == 0
+        assert np.array_equal((out[0] & 1 != 0)[sure], inb[sure])
+        found = sure & (out[0] & 2 != 0)
+        assert np.array_equal(found[sure], hit[sure])
+        assert np.array_equal(out[1][found], kx[found]) and np.array_equal(out[2][found], ky[found])
+        assert found.sum() > len(x) // 100
