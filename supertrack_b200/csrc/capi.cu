@@ -396,6 +396,7 @@ st_status build_tables(st_ctx* c, size_t first, size_t last, bool want_export) {
     D.f_inv_d = 1.0f / D.f_d;
     D.f_r2 = (float)D.r2;
     st::set_integer_geometry(&D);
+    st::set_wrap(&D);
     if (D.flagged) {
       D.cell_cap = next_pow2((uint64_t)2 * (uint64_t)J.track.n);
       D.cell_off = cells_total;

@@ -210,6 +210,7 @@ extern "C" st_status st_superimpose_noalloc(const st_track_view* track, const st
   D.cell_size = (D.cell_nbr8 ? 2.0 : 1.0) * g.sphereDiameter * (1.0 + 0x1p-10);
   D.inv_cell = 1.0 / D.cell_size;
   st::set_integer_geometry(&D);
+  st::set_wrap(&D);
 
   st::HistDev& H = *reinterpret_cast<st::HistDev*>(up + L.hists);
   H.edges = (const double*)(base + L.edges);

@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(1024) k_prep_scan(PrepareParams p) {
     __syncthreads();
   }
   const long long kept = s_carry;
-  const bool many = kept > p.flag_min_kept;
+  const bool many = kept > p.flag_min_kept && !(p.aux[j].flags & kAuxWraps);
   int mode = p.jobs[j].flagged && many ? kWinFlags : kWinNone;
   if (p.jobs[j].layers && many) {
     // the bin counts to first places, and the deposits that lie in bins larger than a window

@@ -86,6 +86,8 @@ struct JobDev {
   int32_t g_shift;
   int32_t g_ns;       // N 2^g_shift
   float g_lo, g_hi;   // squared distance at or below which a deposit hits, above which it misses
+  double wrap_dz;     // |dz| up to which a deposit on a face of the voxel can hit a sphere past the
+                      // lattice (set_wrap), -1: none can
 };
 
 // Integer geometry: x and y of a deposit and the shift of an oversample in units of d / 2^s, rounded
@@ -115,6 +117,52 @@ inline void set_integer_geometry(JobDev* D) {
     D->g_lo = -1.0f;
     D->g_hi = INFINITY;
   }
+}
+
+// Keys of spheres past the lattice. A deposit within a rounding of a face of the voxel can round to
+// lattice index N (or -1), one past the lattice, and hit there when it lies on that sphere's axis.
+// The key of (kx, N, kz) is that of (kx, 0, kz + 1): the reference sums the two as one sphere, although
+// they are a voxel apart, so a job with such a deposit must not be cut into windows. set_wrap finds
+// whether the lattice's roundings allow it and for which z; may_wrap then asks for a deposit with such
+// a z whether some shift (24 bits) puts its x or y there, both in the reference's arithmetic. (The FP32
+// variant's floats wrap at other values, which are not looked for.)
+struct WrapLattice {
+  double HL, L, gSO, d, r2;
+  uint32_t N;
+};
+// Whether coordinate c (after the shift) is in the voxel, past the lattice, and within r of that sphere.
+ST_HD bool wraps(const WrapLattice& g, double c, double* dc) {
+  if (!(fabs(c) < g.HL)) return false;
+  const double a = st_dsub(c, g.gSO);
+  const double k = rint(a / g.d);
+  *dc = st_dsub(st_dmul(k, g.d), a);
+  return (k < 0.0 || k >= (double)g.N) && st_dmul(*dc, *dc) <= g.r2;
+}
+ST_HD bool may_wrap(const WrapLattice& g, int shift_track, double c) {
+  double dc;
+  if (!shift_track) return wraps(g, st_dadd(c, shift_from_uniform(0.5f, g.L, g.HL)), &dc);
+  bool any = false;
+  for (int face = -1; face <= 1; face += 2) {
+    const double m = rint((face * g.HL - c + g.HL) / g.L * 0x1p24);  // the uniform that puts c there
+    for (int k = -2; k <= 2; ++k) {
+      const double u = (m + k) * 0x1p-24;
+      if (u > 0.0 && u <= 1.0)
+        any |= wraps(g, st_dadd(c, shift_from_uniform((float)u, g.L, g.HL)), &dc);
+    }
+  }
+  return any;
+}
+inline void set_wrap(JobDev* D) {
+  const WrapLattice g = {D->HL, D->L, D->gSO, D->d, D->r2, D->N};
+  double dz = -1.0;
+  for (int face = -1; face <= 1; face += 2) {
+    double c = D->HL, dc;
+    for (int k = 0; k < 64; ++k) {  // (the face and the rounding of c - gSO are a few units apart)
+      c = std::nextafter(c, 0.0);
+      if (wraps(g, face * c, &dc)) dz = std::fmax(dz, std::sqrt(g.r2 * (1.0 + 0x1p-50) - dc * dc));
+    }
+  }
+  D->wrap_dz = dz;
 }
 
 // Deposits of a windowed job are processed in windows of consecutive kept deposits: kWindow (two
@@ -162,6 +210,7 @@ struct JobAux {
 };
 constexpr int kAuxNonzero = 1;
 constexpr int kAuxNonfinite = 2;
+constexpr int kAuxWraps = 4;  // some shift can put a deposit past the lattice (may_wrap)
 
 struct HistDev {
   const double* edges;            // nbins + 1 edges
