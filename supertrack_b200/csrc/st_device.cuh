@@ -154,15 +154,13 @@ ST_HD bool may_wrap(const WrapLattice& g, int shift_track, double c) {
 }
 inline void set_wrap(JobDev* D) {
   const WrapLattice g = {D->HL, D->L, D->gSO, D->d, D->r2, D->N};
-  double dz = -1.0;
-  for (int face = -1; face <= 1; face += 2) {
-    double c = D->HL, dc;
-    for (int k = 0; k < 64; ++k) {  // (the face and the rounding of c - gSO are a few units apart)
-      c = std::nextafter(c, 0.0);
-      if (wraps(g, face * c, &dc)) dz = std::fmax(dz, std::sqrt(g.r2 * (1.0 + 0x1p-50) - dc * dc));
-    }
+  D->wrap_dz = -1.0;
+  if (!D->flagged) return;
+  for (int face = -1; face <= 1; face += 2) {  // (farther from the face leaves less for dz)
+    double dc;
+    if (wraps(g, face * std::nextafter(D->HL, 0.0), &dc))
+      D->wrap_dz = std::fmax(D->wrap_dz, std::sqrt(g.r2 * (1.0 + 0x1p-50) - dc * dc));
   }
-  D->wrap_dz = dz;
 }
 
 // Deposits of a windowed job are processed in windows of consecutive kept deposits: kWindow (two
