@@ -229,13 +229,20 @@ struct HistDev {
 // far above its edge even then is added to HBM as a double (sum_span).
 constexpr int kSumBits = 126 - 53;
 inline int keep_bits(const double* edges, int nbins) {
-  int span = 0;
-  for (int b = 0; b < nbins; ++b) {  // (a call without allocation passes here: bits, not ilogb)
-    int64_t lo, hi;
-    std::memcpy(&lo, &edges[b], 8);
-    std::memcpy(&hi, &edges[b + 1], 8);
-    const int e = (int)(lo >> 52), s = (int)(hi >> 52) - e;
-    span = e > 0 && s > span ? s : span;  // (lower edges that are positive normal numbers)
+  const auto exponent = [&](int b) {  // biased; 0 and below: not a positive normal number
+    int64_t bits;
+    std::memcpy(&bits, &edges[b], 8);
+    return (int)(bits >> 52);
+  };
+  int first = 0;
+  while (first < nbins && exponent(first) <= 0) ++first;
+  int span = exponent(nbins) - exponent(first);  // of all such bins: usually little enough
+  if (kSumBits - span < 31) {
+    span = 0;
+    for (int b = first; b < nbins; ++b) {
+      const int s = exponent(b + 1) - exponent(b);
+      span = s > span ? s : span;
+    }
   }
   const int k = kSumBits - span;
   return k < 18 ? 18 : (k > 31 ? 31 : k);

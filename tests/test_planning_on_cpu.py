@@ -200,6 +200,20 @@ def test_kept_sums_stay_below_128_bits(lib, ratio_bits, lower, work):
         assert back == float(y) * spheres
 
 
+@pytest.mark.parametrize("kind,nbins,lower,upper", [
+    ("lin", 3000, 0.01, 300.0), ("log", 500, 0.1, 1e4), ("lin", 1, 1e-13, 1e4), ("lin", 3, 1e-20, 9.0),
+    ("log", 4, 1e-30, 1e30), ("log", 4096, 1e-30, 1e30), ("lin", 10, 0.0, 1.0), ("lin", 7, -3.0, 4.0),
+    ("lin", 2, -1.0, 1.0), ("lin", 1, -2.0, -1.0)])
+def test_keep_bits_of_histograms(lib, kind, nbins, lower, upper):
+    """The widest bin with a positive normal lower edge decides how long a copy is kept."""
+    edges = np.zeros(nbins + 1)
+    _capi.check(_capi.lib().st_hist_edges({"lin": _capi.ST_HIST_LIN, "log": _capi.ST_HIST_LOG}[kind], nbins, lower, upper,
+                                          _ptr(edges)), "st_hist_edges")
+    e = np.frexp(edges)[1]
+    wide = [int(b - a) for a, b, lo in zip(e, e[1:], edges) if lo >= 2.0 ** -1022]
+    assert lib.keep_bits(_ptr(edges), nbins) == min(31, max(18, 73 - max(wide, default=0)))
+
+
 @pytest.mark.parametrize("win_tiles", [32, 64])
 @pytest.mark.parametrize("m", [1, 3, 4, 5, 8, 100])
 def test_window_list(lib, m, win_tiles):
