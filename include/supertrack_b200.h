@@ -184,7 +184,9 @@ ST_API st_status st_ctx_set_tuning(st_ctx* ctx, int64_t item_cost, int32_t grid)
  *   sort_deposits      order of the kept deposits: 0 source order. 1: the jobs that qualify for
  *                      window boundary flags (see flag_min_kept) are ordered by z layer instead
  *                      and run in windows of whole layers, which share no sphere (a track across
- *                      z, with most deposits in a few layers, keeps the flags); their prepare
+ *                      z, with most deposits in a few layers, keeps the flags where layers would
+ *                      spill or leave CTAs without work; a track with a deposit that can hit one
+ *                      sphere past the lattice runs without windows); their prepare
  *                      blocks (1024 source deposits) write their kept deposits grouped by
  *                      d-cell, so that deposits of one sphere arrive together in the fused
  *                      kernel. 2: the blocks of all other jobs are grouped too. Results do not
